@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/nmag_gpu.h"
+#include "nd_solve.h"
 
 namespace nmg {
 
@@ -150,6 +151,27 @@ struct TcState {
   alignas(64) unsigned char mapX[128];
 };
 
+// One Poisson system's direct solver (nd_solve.cu): the separator tree, its
+// factor, the sweeps' task lists and the matrix in elimination order.
+struct NdSystem {
+  bool ready = false;
+  int n = 0, nlev = 0, grid = 1;  // active nodes, tree levels, blocks of a solve
+  long long entries = 0, nu = 0;  // factor entries; upward-sweep vector entries
+  DevBuf<NdFront> front;
+  DevBuf<NdLevel> phase;
+  DevBuf<NdTask> task;
+  DevBuf<int32_t> bnd, map, perm, prow, pcol;   // perm: position of each node (-1: fixed), then node of each position
+  DevBuf<double> pK, f64, one, kone;   // one, kone: the Neumann sweeps' answer to b = 1 and K times it
+  DevBuf<float> f32;
+};
+struct NdSolver {
+  NdSystem sys[2];                // 0: Neumann, 1: Dirichlet
+  bool tried = false;             // nd_prepare has run
+  int evals = 0;                  // demag evaluations so far
+  DevBuf<double> u, d, xw, r, part;   // member-minor work vectors, reduction partials
+  DevBuf<unsigned> bar;           // barrier counter, blocks that left (both zero between launches)
+};
+
 // Several magnetic materials (nmag_lam.py:183-330): every material X has its
 // own m_X on its sites -- the nodes of the simplices of the regions carrying
 // X.  The handle's mesh is then the site mesh, the disjoint union of the
@@ -278,6 +300,7 @@ struct nmg_handle {
   nmg::AnisPoly ap;
   nmg::Stt stt;
   nmg::DevBuf<double> pin;      // per-node factor of dm/dt and of the Jacobian rows (null: 1 everywhere)
+  nmg::NdSolver nd;             // direct Poisson solves
   nmg::TcState tc;              // tensor-core BEM product (bem_precision 3)
   nmg::Sites sites;             // several materials: the site layout (n_mats == 0: one material)
   nmg_handle *pot = nullptr;    // several materials: the handle of the potential mesh (owns BEM, CG)
@@ -345,6 +368,14 @@ int demag_response_sites(nmg_handle *h, const double *d_v);
 // at rtol; jac_prepare allocates J (zeroed) for P's workspace once
 int jac_prepare(nmg_handle *P, JacDemag &J);
 int jac_demag_solve(nmg_handle *P, JacDemag &J, double rtol);
+// ---- nd_solve.cu (direct Poisson solves) ----
+// nd_prepare factors, once per handle, the systems the solver applies to
+// (nd_available); nd_solve: nm <= kChunk right-hand sides (member m at b + m * N)
+// to max(rtol |b|, atol).
+int nd_prepare(nmg_handle *h);
+bool nd_available(const nmg_handle *h, int mode);
+int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32);
+void nd_reset_barrier(nmg_handle *h);   // after a launch whose barrier gave up
 // ---- bem_tc.cu ----
 int bem_tc_setup(nmg_handle *h, std::string &err);
 int bem_tc(nmg_handle *h, const double *x, double *y, int R);   // Y = B X, R member-major right-hand sides

@@ -1261,6 +1261,7 @@ void ts_destroy(Integrator *I) {
 
 int ts_init(nmg_handle *h, double t0) {
   Integrator &I = *h->ts;
+  if (int rc = nd_prepare(h)) return rc;
   I.tn = t0; I.q = 1; I.L = 2; I.qwait = I.L; I.qprime = 1;
   I.nst = I.nfe = I.nni = I.nli = I.ncfn = I.netf = I.nsetups = I.npe = I.nps = I.njv = 0;
   I.nstlp = I.nstlpre = 0;
@@ -1328,6 +1329,8 @@ int ts_advance(nmg_handle *h, double tout, int exact_tstop, int64_t max_steps, d
 // Classical RK4 with fixed dt on device vectors (differentiation form forward).
 int rk4_device(nmg_handle *h, double *d_m, double dt, int nsteps) {
   const int n = 3 * h->mesh.N * h->nrep;
+  if (nsteps > 0)
+    if (int rc = nd_prepare(h)) return rc;
   DevBuf<double> buf;
   if (buf.alloc(5 * (size_t)n)) return 100;
   double *k1 = buf.p, *k2 = k1 + n, *k3 = k2 + n, *k4 = k3 + n, *y = k4 + n;

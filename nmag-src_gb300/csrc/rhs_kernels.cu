@@ -2493,6 +2493,7 @@ void wait_basis_factor(nmg_handle *h, int ev_slot) {
 }
 
 int run_cg(nmg_handle *h, int mode, const double *b, double *x, double rtol, double atol, int maxits) {
+  if (nd_available(h, mode & 1)) return nd_solve(h, mode & 1, 1, b, x, rtol, atol, false);
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   CGArgs a;
@@ -2536,6 +2537,8 @@ int run_cg(nmg_handle *h, int mode, const double *b, double *x, double rtol, dou
 // mixed precision, 0 FP64, -1 the handle's forward choice.
 int run_cgm(nmg_handle *h, int mode, int c0, const double *b, double *x, int nm, double rtol, double atol,
             int maxits, int bslot = -1, int mp_sel = -1) {
+  if (nd_available(h, mode))
+    return nd_solve(h, mode, nm, b, x, rtol, atol, mp_sel >= 0 ? mp_sel == 1 : h->opt.cg_precision == 1);
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   CGArgs a;
@@ -3010,6 +3013,7 @@ int check_device_error(nmg_handle *h, const char *where) {
   }
   if (derr) {
     cudaMemsetAsync(h->ws.err.p, 0, sizeof(int), h->stream);
+    if (derr & ERR_BARRIER) nd_reset_barrier(h);
     if (derr & ERR_BARRIER) h->last_error = std::string(where) + ": grid barrier timed out";
     else if (derr & ERR_NONFINITE) h->last_error = std::string(where) + ": solver produced non-finite values";
     else if (derr & ERR_CG_MAXITS) h->last_error = std::string(where) + ": CG reached its iteration limit";
@@ -3023,6 +3027,8 @@ int check_device_error(nmg_handle *h, const char *where) {
 // potential W.phi: Neumann solve, boundary gather, BEM product, Dirichlet
 // load and solve, phi = phi1 + phi2 (nmag_lam.py:740-760).
 int demag_from_rho(nmg_handle *h) {
+  if (++h->nd.evals >= kNdEvals)
+    if (int rc = nd_prepare(h)) return rc;
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   cudaStream_t s = h->stream;
