@@ -8,8 +8,12 @@
 // particle).  One CTA owns one particle at a time: it takes the next particle
 // from a queue ordered by decreasing cost (nb^2 + CG work) and runs whole
 // integrator steps for it with block-level synchronisation only, so particles
-// of 125 and 9,261 nodes share the GPU without grid barriers.  Inside a CTA
-// the right-hand side is the single path's pipeline (nmag_lam.py:734-832):
+// of 125 and 9,261 nodes share the GPU without grid barriers.  A particle that
+// one CTA would still be working on when the rest of the batch is done belongs
+// to a team instead: the kTeam CTAs of a thread-block cluster share its rows
+// and meet at the cluster's hardware barrier (every cluster takes team
+// particles first, then its CTAs take the small ones by themselves).
+// The right-hand side is the single path's pipeline (nmag_lam.py:734-832):
 // rho = -Ms D m, Neumann Jacobi-PCG, BEM product (warp per row, x in shared
 // memory), Dirichlet Jacobi-PCG, fused H_eff + LLG.  Time integration is the
 // embedded Bogacki-Shampine 3(2) pair with per-particle step control (FSAL),
@@ -24,6 +28,8 @@
 #include <numeric>
 #include <string>
 #include <vector>
+
+#include <cooperative_groups.h>
 
 #include "nmg_internal.h"
 
@@ -42,6 +48,11 @@ struct PDesc {
   int pad;
 };
 
+// CTAs of a team: the portable cluster size, and the warps of the 256-thread
+// CTA whose sums a team reproduces bit for bit (team_cg).
+constexpr int kTeam = 8;
+constexpr int kTeamThreads = 32 * kTeam;
+
 struct PState {
   double t, dt, hmag, maxdmdt;
   int stage, done, conv, have_k1;
@@ -53,12 +64,13 @@ struct BatchArgs {
   int P, n_stages, cg_maxits, adaptive;
   int integrator, krylov_maxits;   // 0: Bogacki-Shampine 3(2); 1: ROS2 (linearly implicit)
   double hmax, rtol, atol, cg_rtol, stop_dmdt, dt_max;
-  const int *order;
-  int *queue;                      // next queue position (reset before each launch)
+  const int *order;                // team particles first (n_team of them), each part by decreasing cost
+  int n_team;
+  int *queue;                      // next queue positions: team particles, the others (reset before each launch)
   const PDesc *desc;
   PState *st;
   const int32_t *row_ptr, *col_idx, *diag, *b_of_node, *node_of_b;
-  const double *K, *Gx, *Gy, *Gz, *Dx, *Dy, *Dz, *vol;
+  const double *K, *Gx, *Gy, *Gz, *Dx, *Dy, *Dz, *vol, *dinv;
   const float *bem;
   double *m, *k0, *k1, *k2, *k3, *y, *phi1, *phi2, *rho, *rhs2, *cr, *cz, *cp, *cq, *b2, *hout;
   // ROS2: field at the step's start, 3x3 block inverses of W, Krylov vectors (3N per particle)
@@ -91,6 +103,52 @@ __device__ __forceinline__ void bsum2(double &a, double &b, double *sm) {
   b = tb;
 }
 
+// The CTAs working on one particle.
+struct Team {
+  int rank, size;
+  int phase;   // parity of the exchange slots
+};
+
+__device__ __forceinline__ void tsync(const Team &t) {
+  if (t.size == 1) __syncthreads();
+  else asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
+// Team-wide sums of two values (or maximum of a), the same in every thread:
+// each CTA's share goes to every CTA's slots through distributed shared
+// memory.  sm: block scratch; ex: 2 x kTeam x 2 exchange slots of this CTA.
+template <bool MAX>
+__device__ __forceinline__ void treduce(Team &t, double &a, double &b, double *sm, double *ex) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  a = MAX ? wmax(a) : wsum(a);
+  if (!MAX) b = wsum(b);
+  if (lane == 0) { sm[w] = a; sm[kMaxWarps + w] = b; }
+  __syncthreads();
+  double ta = 0.0, tb = 0.0;
+  for (int q = 0; q < nw; ++q) {
+    ta = MAX ? fmax(ta, sm[q]) : ta + sm[q];
+    if (!MAX) tb += sm[kMaxWarps + q];
+  }
+  __syncthreads();
+  if (t.size > 1) {
+    double *slot = ex + t.phase * 2 * kTeam;
+    t.phase ^= 1;
+    if ((int)threadIdx.x < t.size) {
+      double *r = cooperative_groups::this_cluster().map_shared_rank(slot, threadIdx.x);
+      r[2 * t.rank] = ta;
+      r[2 * t.rank + 1] = tb;
+    }
+    tsync(t);
+    ta = tb = 0.0;
+    for (int q = 0; q < t.size; ++q) {
+      ta = MAX ? fmax(ta, slot[2 * q]) : ta + slot[2 * q];
+      if (!MAX) tb += slot[2 * q + 1];
+    }
+  }
+  a = ta;
+  b = tb;
+}
+
 __device__ __forceinline__ double bmax(double a, double *sm) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   a = wmax(a);
@@ -105,7 +163,7 @@ __device__ __forceinline__ double bmax(double a, double *sm) {
 struct PView {   // one particle's slices
   int N, nb, ld;
   const int32_t *rp, *ci, *diag, *bon, *nob;
-  const double *K, *Gx, *Gy, *Gz, *Dx, *Dy, *Dz, *vol;
+  const double *K, *Gx, *Gy, *Gz, *Dx, *Dy, *Dz, *vol, *dinv;   // dinv: 1 / K_ii
   const float *bem;
   double *phi1, *phi2, *rho, *rhs2, *cr, *cz, *cp, *cq, *b2;
 };
@@ -121,6 +179,7 @@ __device__ PView view(const BatchArgs &a, int p, const PDesc &d) {
   v.K = a.K + d.onz; v.Gx = a.Gx + d.onz; v.Gy = a.Gy + d.onz; v.Gz = a.Gz + d.onz;
   v.Dx = a.Dx + d.onz; v.Dy = a.Dy + d.onz; v.Dz = a.Dz + d.onz;
   v.vol = a.vol + d.on;
+  v.dinv = a.dinv + d.on;
   v.bem = a.bem + d.obem;
   v.phi1 = a.phi1 + d.on; v.phi2 = a.phi2 + d.on; v.rho = a.rho + d.on; v.rhs2 = a.rhs2 + d.on;
   v.cr = a.cr + d.on; v.cz = a.cz + d.on; v.cp = a.cp + d.on; v.cq = a.cq + d.on;
@@ -161,7 +220,7 @@ __device__ int block_cg(const PView &v, int mode, const double *b, double *x, do
   for (int i = tid; i < N; i += nt) {
     const double bi = b[i] - mean;
     const double ri = bi - apply_row(v, mode, i, x);
-    const double di = (mode == 1 && v.bon[i] >= 0) ? 1.0 : 1.0 / v.K[v.diag[i]];
+    const double di = (mode == 1 && v.bon[i] >= 0) ? 1.0 : v.dinv[i];
     v.cr[i] = ri;
     v.cz[i] = di * ri;
     v.cp[i] = di * ri;
@@ -188,7 +247,7 @@ __device__ int block_cg(const PView &v, int mode, const double *b, double *x, do
     for (int i = tid; i < N; i += nt) {
       x[i] += alpha * v.cp[i];
       const double ri = v.cr[i] - alpha * v.cq[i];
-      const double di = (mode == 1 && v.bon[i] >= 0) ? 1.0 : 1.0 / v.K[v.diag[i]];
+      const double di = (mode == 1 && v.bon[i] >= 0) ? 1.0 : v.dinv[i];
       v.cr[i] = ri;
       v.cz[i] = di * ri;
       rzn += ri * di * ri;
@@ -212,10 +271,106 @@ __device__ int block_cg(const PView &v, int mode, const double *b, double *x, do
   return it;
 }
 
-// dm/dt = f(y) for one particle (block); H_total to hout when given.
+// block_cg by a team, bit for bit what one CTA of kTeamThreads threads gives
+// (the adaptive steps follow last-bit changes of the slopes: 3e5 times larger
+// in the step size at a tolerance of 1e-7, so that a team's particle takes the
+// steps it would take alone).  CTA r has the rows of that CTA's warp r, i mod
+// kTeamThreads in [32 r, 32 r + 32), all its warps sharing them by blocks of
+// 32; a sum is then one warp's chain over the blocks in order, as the warp of
+// the single CTA adds them, the butterfly, and the warps' sums in order.
+// 9,261 nodes: 125 us an iteration in one CTA (with a division per row, which is
+// gone too), 28 here.
+__device__ int team_cg(const PView &v, int mode, const double *b, double *x, double rtol, int maxits, Team &T,
+                       double *ex, bool *failed) {
+  const int N = v.N, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int first = 32 * T.rank + lane;   // row of block c: first + kTeamThreads * c
+  // two chains over this CTA's rows, one by warp 0 (f), one by warp 1 (g), and
+  // their sums over the team
+  auto sums = [&](auto f, auto g, double &sf, double &sg) {
+    __syncthreads();
+    double *slot = ex + T.phase * 2 * kTeam;
+    T.phase ^= 1;
+    if (w < 2) {
+      double acc = 0.0;
+      if (w == 0) {
+#pragma unroll 8
+        for (int i = first; i < N; i += kTeamThreads) acc = f(i, acc);
+      } else {
+#pragma unroll 8
+        for (int i = first; i < N; i += kTeamThreads) acc = g(i, acc);
+      }
+      acc = wsum(acc);
+      if (lane < kTeam) cooperative_groups::this_cluster().map_shared_rank(slot, lane)[2 * T.rank + w] = acc;
+    }
+    tsync(T);
+    sf = sg = 0.0;
+    for (int q = 0; q < kTeam; ++q) { sf += slot[2 * q]; sg += slot[2 * q + 1]; }
+  };
+  auto none = [](int, double acc) { return acc; };
+  double mean = 0.0, dummy;
+  if (mode == 0) {
+    double s;
+    sums([&](int i, double acc) { return acc + b[i]; }, none, s, dummy);
+    mean = s / N;
+  } else {
+    for (int i = first + kTeamThreads * w; i < N; i += kTeamThreads * kTeam)
+      if (v.bon[i] >= 0) x[i] = b[i];
+    tsync(T);
+  }
+  for (int i = first + kTeamThreads * w; i < N; i += kTeamThreads * kTeam) {
+    const double ri = (b[i] - mean) - apply_row(v, mode, i, x);
+    const double di = (mode == 1 && v.bon[i] >= 0) ? 1.0 : v.dinv[i];
+    v.cr[i] = ri;
+    v.cz[i] = di * ri;
+    v.cp[i] = di * ri;
+  }
+  double bb, rz, rr;
+  sums([&](int i, double acc) { const double bi = b[i] - mean; return fma(bi, bi, acc); },
+       [&](int i, double acc) { return fma(v.cz[i], v.cr[i], acc); }, bb, rz);
+  const double tol = fmax(rtol * sqrt(bb), 1e-300);
+  sums([&](int i, double acc) { return fma(v.cr[i], v.cr[i], acc); }, none, rr, dummy);
+  int it = 0;
+  while (sqrt(rr) > tol) {
+    if (it >= maxits || !(rr == rr)) { *failed = true; break; }
+    for (int i = first + kTeamThreads * w; i < N; i += kTeamThreads * kTeam) v.cq[i] = apply_row(v, mode, i, v.cp);
+    double pq;
+    sums([&](int i, double acc) { return fma(v.cp[i], v.cq[i], acc); }, none, pq, dummy);
+    const double alpha = rz / pq;
+    for (int i = first + kTeamThreads * w; i < N; i += kTeamThreads * kTeam) {
+      x[i] = fma(alpha, v.cp[i], x[i]);
+      const double ri = fma(-alpha, v.cq[i], v.cr[i]);
+      const double di = (mode == 1 && v.bon[i] >= 0) ? 1.0 : v.dinv[i];
+      v.cr[i] = ri;
+      v.cz[i] = di * ri;
+    }
+    double rzn, rrn;
+    sums([&](int i, double acc) { return fma(v.cz[i], v.cr[i], acc); },
+         [&](int i, double acc) { return fma(v.cr[i], v.cr[i], acc); }, rzn, rrn);
+    const double beta = rzn / rz;
+    rz = rzn;
+    rr = rrn;
+    for (int i = first + kTeamThreads * w; i < N; i += kTeamThreads * kTeam) v.cp[i] = fma(beta, v.cp[i], v.cz[i]);
+    tsync(T);
+    ++it;
+  }
+  if (mode == 0) {
+    double s;
+    sums([&](int i, double acc) { return acc + x[i]; }, none, s, dummy);
+    for (int i = first + kTeamThreads * w; i < N; i += kTeamThreads * kTeam) x[i] -= s / N;
+  }
+  tsync(T);
+  return it;
+}
+
+// dm/dt = f(y) for one particle (its team); H_total to hout when given.
 __device__ void prhs(const BatchArgs &a, int p, const PDesc &d, const PView &v, double hmag, const double *y,
-                     double *out, double *hout, double *sm, float *xs, PState &st, bool *failed) {
-  const int N = v.N, tid = threadIdx.x, nt = blockDim.x;
+                     double *out, double *hout, double *sm, float *xs, PState &st, bool *failed, Team &T,
+                     double *ex) {
+  const int N = v.N, tid = T.rank * blockDim.x + threadIdx.x, nt = T.size * blockDim.x;
+  auto poisson = [&](int mode, const double *b, double *x) {
+    st.cg_iters += T.size > 1 ? team_cg(v, mode, b, x, a.cg_rtol, a.cg_maxits, T, ex, failed)
+                              : block_cg(v, mode, b, x, a.cg_rtol, a.cg_maxits, sm, failed);
+  };
   // rho = -Ms D y
   for (int i = tid; i < N; i += nt) {
     double s = 0.0;
@@ -225,13 +380,13 @@ __device__ void prhs(const BatchArgs &a, int p, const PDesc &d, const PView &v, 
     }
     v.rho[i] = -(d.Ms * s);
   }
-  __syncthreads();
-  st.cg_iters += block_cg(v, 0, v.rho, v.phi1, a.cg_rtol, a.cg_maxits, sm, failed);
+  tsync(T);
+  poisson(0, v.rho, v.phi1);
   // BEM product phi2b = B phi1b (FP32 matrix and x, FP64 row sums)
-  for (int j = tid; j < v.ld; j += nt) xs[j] = j < v.nb ? (float)v.phi1[v.nob[j]] : 0.0f;
+  for (int j = threadIdx.x; j < v.ld; j += blockDim.x) xs[j] = j < v.nb ? (float)v.phi1[v.nob[j]] : 0.0f;
   __syncthreads();
   {
-    const int lane = tid & 31, w = tid >> 5, nw = nt >> 5;
+    const int lane = threadIdx.x & 31, w = tid >> 5, nw = nt >> 5;
     for (int r = w; r < v.nb; r += nw) {
       const float4 *row = reinterpret_cast<const float4 *>(v.bem + (size_t)r * v.ld);
       const float4 *x4 = reinterpret_cast<const float4 *>(xs);
@@ -245,7 +400,7 @@ __device__ void prhs(const BatchArgs &a, int p, const PDesc &d, const PView &v, 
       if (lane == 0) v.b2[r] = s;
     }
   }
-  __syncthreads();
+  tsync(T);
   // Dirichlet right-hand side (op_load_DBC): interior -K_IB phi2b, boundary phi2b
   for (int i = tid; i < N; i += nt) {
     const int bi = v.bon[i];
@@ -257,8 +412,8 @@ __device__ void prhs(const BatchArgs &a, int p, const PDesc &d, const PView &v, 
     }
     v.rhs2[i] = -s;
   }
-  __syncthreads();
-  st.cg_iters += block_cg(v, 1, v.rhs2, v.phi2, a.cg_rtol, a.cg_maxits, sm, failed);
+  tsync(T);
+  poisson(1, v.rhs2, v.phi2);
   // fused H_eff + LLG
   for (int i = tid; i < N; i += nt) {
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, g0 = 0.0, g1 = 0.0, g2 = 0.0;
@@ -288,7 +443,7 @@ __device__ void prhs(const BatchArgs &a, int p, const PDesc &d, const PView &v, 
       if (hout) hout[3 * (size_t)i + c] = H[c];
     }
   }
-  __syncthreads();
+  tsync(T);
   st.rhs++;
 }
 
@@ -298,29 +453,30 @@ __device__ __forceinline__ double stage_field(const BatchArgs &a, int stage) {
 
 // Up to d.steps_cap Bogacki-Shampine steps (with the hysteresis stage logic)
 // for particle p.
-__device__ void particle_run(const BatchArgs &a, int p, double *sm, float *xs, PState &st) {
+__device__ void particle_run(const BatchArgs &a, int p, double *sm, float *xs, PState &st, Team &T,
+                             double *ex) {
   const PDesc d = a.desc[p];
   const PView v = view(a, p, d);
-  const int n3 = 3 * d.N, tid = threadIdx.x, nt = blockDim.x;
+  const int n3 = 3 * d.N, tid = T.rank * blockDim.x + threadIdx.x, nt = T.size * blockDim.x;
   const size_t o3 = 3 * (size_t)d.on;
   double *m = a.m + o3, *k0 = a.k0 + o3, *k1 = a.k1 + o3, *k2 = a.k2 + o3, *k3 = a.k3 + o3, *y = a.y + o3;
   bool failed = false;
   for (int s = 0; s < d.steps_cap && !st.done; ++s) {
     if (!st.have_k1) {
-      prhs(a, p, d, v, st.hmag, m, k0, nullptr, sm, xs, st, &failed);
+      prhs(a, p, d, v, st.hmag, m, k0, nullptr, sm, xs, st, &failed, T, ex);
       st.have_k1 = 1;
     }
     const double dt = st.dt;
     for (int i = tid; i < n3; i += nt) y[i] = m[i] + 0.5 * dt * k0[i];
-    __syncthreads();
-    prhs(a, p, d, v, st.hmag, y, k1, nullptr, sm, xs, st, &failed);
+    tsync(T);
+    prhs(a, p, d, v, st.hmag, y, k1, nullptr, sm, xs, st, &failed, T, ex);
     for (int i = tid; i < n3; i += nt) y[i] = m[i] + 0.75 * dt * k1[i];
-    __syncthreads();
-    prhs(a, p, d, v, st.hmag, y, k2, nullptr, sm, xs, st, &failed);
+    tsync(T);
+    prhs(a, p, d, v, st.hmag, y, k2, nullptr, sm, xs, st, &failed, T, ex);
     for (int i = tid; i < n3; i += nt)
       y[i] = m[i] + dt * (((2.0 / 9.0) * k0[i] + (1.0 / 3.0) * k1[i]) + (4.0 / 9.0) * k2[i]);
-    __syncthreads();
-    prhs(a, p, d, v, st.hmag, y, k3, nullptr, sm, xs, st, &failed);
+    tsync(T);
+    prhs(a, p, d, v, st.hmag, y, k3, nullptr, sm, xs, st, &failed, T, ex);
     double en = 0.0;
     if (a.adaptive) {
       for (int i = tid; i < n3; i += nt) {
@@ -328,7 +484,8 @@ __device__ void particle_run(const BatchArgs &a, int p, double *sm, float *xs, P
                                (4.0 / 9.0 - 1.0 / 3.0) * k2[i]) - 0.125 * k3[i]);
         en = fmax(en, fabs(e) / (a.atol + a.rtol * fmax(fabs(m[i]), fabs(y[i]))));
       }
-      en = bmax(en, sm);
+      double none = 0.0;
+      treduce<true>(T, en, none, sm, ex);
     }
     if (failed || !(en == en)) {
       if (tid == 0) atomicOr(a.err, ERR_NONFINITE);
@@ -345,7 +502,8 @@ __device__ void particle_run(const BatchArgs &a, int p, double *sm, float *xs, P
         const double *f = k3 + 3 * (size_t)i;
         mx = fmax(mx, sqrt((f[0] * f[0] + f[1] * f[1]) + f[2] * f[2]));
       }
-      mx = bmax(mx, sm);
+      double none = 0.0;
+      treduce<true>(T, mx, none, sm, ex);
       st.t += dt;
       st.steps++;
       st.maxdmdt = mx;
@@ -363,7 +521,7 @@ __device__ void particle_run(const BatchArgs &a, int p, double *sm, float *xs, P
       const double fac = en > 0.0 ? 0.9 * pow(en, -1.0 / 3.0) : 5.0;
       st.dt = fmin(a.dt_max, dt * fmin(5.0, fmax(0.2, fac)));
     }
-    __syncthreads();
+    tsync(T);
   }
 }
 
@@ -532,7 +690,9 @@ __device__ int block_bicgstab(const PView &v, const PDesc &d, const double *m, c
 }
 
 // Up to d.steps_cap ROS2 steps (with the hysteresis stage logic) for particle p.
-__device__ void particle_run_ros2(const BatchArgs &a, int p, double *sm, float *xs, PState &st) {
+__device__ void particle_run_ros2(const BatchArgs &a, int p, double *sm, float *xs, PState &st,
+                                  double *ex) {
+  Team T = {0, 1, 0};
   const PDesc d = a.desc[p];
   const PView v = view(a, p, d);
   const int n3 = 3 * d.N, N = d.N, tid = threadIdx.x, nt = blockDim.x;
@@ -544,7 +704,7 @@ __device__ void particle_run_ros2(const BatchArgs &a, int p, double *sm, float *
   bool failed = false;
   for (int s = 0; s < d.steps_cap && !st.done; ++s) {
     if (!st.have_k1) {   // f and H at the step's start (after a new field of the sweep)
-      prhs(a, p, d, v, st.hmag, m, f0, H, sm, xs, st, &failed);
+      prhs(a, p, d, v, st.hmag, m, f0, H, sm, xs, st, &failed, T, ex);
       st.have_k1 = 1;
     }
     const double tau = st.dt, gt = kRos2Gamma * tau;
@@ -554,7 +714,7 @@ __device__ void particle_run_ros2(const BatchArgs &a, int p, double *sm, float *
     st.krylov_iters += block_bicgstab(v, d, m, H, gt, Pinv, f0, k1, krtol, a.krylov_maxits, K, sm, &failed);
     for (int o = tid; o < n3; o += nt) y[o] = m[o] + tau * k1[o];
     __syncthreads();
-    prhs(a, p, d, v, st.hmag, y, f1, nullptr, sm, xs, st, &failed);
+    prhs(a, p, d, v, st.hmag, y, f1, nullptr, sm, xs, st, &failed, T, ex);
     for (int o = tid; o < n3; o += nt) {
       f1[o] -= 2.0 * k1[o];
       k2[o] = f1[o];
@@ -577,7 +737,7 @@ __device__ void particle_run_ros2(const BatchArgs &a, int p, double *sm, float *
     if (en <= 1.0) {   // accept: m <- y, then f and H there (the next step's start)
       for (int o = tid; o < n3; o += nt) m[o] = y[o];
       __syncthreads();
-      prhs(a, p, d, v, st.hmag, m, f0, H, sm, xs, st, &failed);
+      prhs(a, p, d, v, st.hmag, m, f0, H, sm, xs, st, &failed, T, ex);
       double mx = 0.0;
       for (int i = tid; i < N; i += nt) {
         const double *f = f0 + 3 * (size_t)i;
@@ -605,52 +765,92 @@ __device__ void particle_run_ros2(const BatchArgs &a, int p, double *sm, float *
   }
 }
 
-__global__ void k_batch_run(BatchArgs a) {
+// The next team particle (every CTA of the cluster learns it), or -1.
+__device__ int next_team_particle(const BatchArgs &a, const Team &T, int *sp) {
+  if (T.rank == 0 && threadIdx.x == 0) {
+    const int q = atomicAdd(a.queue, 1), p = q < a.n_team ? a.order[q] : -1;
+    for (int r = 0; r < T.size; ++r) *cooperative_groups::this_cluster().map_shared_rank(sp, r) = p;
+  }
+  tsync(T);
+  const int p = *sp;
+  tsync(T);   // everyone has read it
+  return p;
+}
+__device__ int next_particle(const BatchArgs &a, int *sp) {
+  if (threadIdx.x == 0) {
+    const int q = a.n_team + atomicAdd(a.queue + 1, 1);
+    *sp = q < a.P ? a.order[q] : -1;
+  }
+  __syncthreads();
+  const int p = *sp;
+  __syncthreads();
+  return p;
+}
+__device__ Team cluster_team() {
+  unsigned rank, size;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+  return {(int)rank, (int)size, 0};
+}
+
+__global__ void __launch_bounds__(352) k_batch_run(BatchArgs a) {   // 352: the largest CTA a schedule may choose
   extern __shared__ float xs[];
-  __shared__ double sm[2 * kMaxWarps];
+  __shared__ double sm[2 * kMaxWarps], ex[4 * kTeam];
   __shared__ int sp;
-  __shared__ PState st;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const int q = atomicAdd(a.queue, 1);
-      sp = q < a.P ? a.order[q] : -1;
-      if (sp >= 0) st = a.st[sp];
+  // every thread works on a private copy of a particle's scalars; one is stored
+  if (a.n_team > 0) {
+    Team T = cluster_team();
+    for (;;) {
+      const int p = next_team_particle(a, T, &sp);
+      if (p < 0) break;
+      PState mine = a.st[p];
+      if (!mine.done) particle_run(a, p, sm, xs, mine, T, ex);
+      tsync(T);   // every CTA has read the state it replaces
+      if (T.rank == 0 && threadIdx.x == 0) a.st[p] = mine;
     }
-    __syncthreads();
-    const int p = sp;
+  }
+  Team T = {0, 1, 0};
+  for (;;) {
+    const int p = next_particle(a, &sp);
     if (p < 0) break;
-    // every thread works on a private copy of the scalars; thread 0's is stored
-    PState mine = st;
+    PState mine = a.st[p];
     if (!mine.done) {
-      if (a.integrator == 1) particle_run_ros2(a, p, sm, xs, mine);
-      else particle_run(a, p, sm, xs, mine);
+      if (a.integrator == 1) particle_run_ros2(a, p, sm, xs, mine, ex);
+      else particle_run(a, p, sm, xs, mine, T, ex);
     }
     __syncthreads();
     if (threadIdx.x == 0) a.st[p] = mine;
-    __syncthreads();
   }
 }
 
 // One RHS evaluation per particle at its current m and stage field.
-__global__ void k_batch_eval(BatchArgs a, double *dmdt) {
+__global__ void __launch_bounds__(352) k_batch_eval(BatchArgs a, double *dmdt) {
   extern __shared__ float xs[];
-  __shared__ double sm[2 * kMaxWarps];
+  __shared__ double sm[2 * kMaxWarps], ex[4 * kTeam];
   __shared__ int sp;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const int q = atomicAdd(a.queue, 1);
-      sp = q < a.P ? a.order[q] : -1;
-    }
-    __syncthreads();
-    const int p = sp;
-    if (p < 0) break;
+  auto eval = [&](int p, Team &T) {
     const PDesc d = a.desc[p];
     const PView v = view(a, p, d);
     PState st = a.st[p];
     bool failed = false;
     prhs(a, p, d, v, st.hmag, a.m + 3 * (size_t)d.on, dmdt + 3 * (size_t)d.on, a.hout + 3 * (size_t)d.on, sm, xs,
-         st, &failed);
-    if (failed && threadIdx.x == 0) atomicOr(a.err, ERR_CG_MAXITS);
+         st, &failed, T, ex);
+    if (failed && T.rank == 0 && threadIdx.x == 0) atomicOr(a.err, ERR_CG_MAXITS);
+  };
+  if (a.n_team > 0) {
+    Team T = cluster_team();
+    for (;;) {
+      const int p = next_team_particle(a, T, &sp);
+      if (p < 0) break;
+      eval(p, T);
+      tsync(T);
+    }
+  }
+  Team T = {0, 1, 0};
+  for (;;) {
+    const int p = next_particle(a, &sp);
+    if (p < 0) break;
+    eval(p, T);
     __syncthreads();
   }
 }
@@ -668,13 +868,14 @@ struct nmg_batch {
   int ld_max = 8;
   long long Ntot = 0;
   nmg::DevBuf<int32_t> row_ptr, col_idx, diag, b_of_node, node_of_b, order, queue;
-  nmg::DevBuf<double> K, Gx, Gy, Gz, Dx, Dy, Dz, vol;
+  nmg::DevBuf<double> K, Gx, Gy, Gz, Dx, Dy, Dz, vol, dinv;
   nmg::DevBuf<float> bem;
   nmg::DevBuf<double> m, k0, k1, k2, k3, y, phi1, phi2, rho, rhs2, cr, cz, cp, cq, b2, hout, dmdt;
   nmg::DevBuf<double> hn, pinv, kr, krh, kp, kv, ks, kt, kph, ksh;   // ROS2 integrator only
   nmg::DevBuf<nmg::PDesc> desc;
   nmg::DevBuf<nmg::PState> st;
   nmg::DevBuf<int> err;
+  int n_large = 0, n_team = 0;   // particles for teams; of them those the schedule gives to teams
   int threads = 256;
   double budget = 0.0;
   int blocks = 0;
@@ -705,8 +906,9 @@ nmg::BatchArgs nmg_batch::args() const {
   a.hmax = opt.h_max; a.rtol = opt.rtol; a.atol = opt.atol; a.cg_rtol = opt.cg_rtol;
   a.stop_dmdt = opt.stop_dmdt; a.dt_max = opt.dt_max;
   a.order = order; a.queue = queue; a.desc = desc; a.st = st;
+  a.n_team = n_team;
   a.row_ptr = row_ptr; a.col_idx = col_idx; a.diag = diag; a.b_of_node = b_of_node; a.node_of_b = node_of_b;
-  a.K = K; a.Gx = Gx; a.Gy = Gy; a.Gz = Gz; a.Dx = Dx; a.Dy = Dy; a.Dz = Dz; a.vol = vol; a.bem = bem;
+  a.K = K; a.Gx = Gx; a.Gy = Gy; a.Gz = Gz; a.Dx = Dx; a.Dy = Dy; a.Dz = Dz; a.vol = vol; a.dinv = dinv; a.bem = bem;
   a.m = m; a.k0 = k0; a.k1 = k1; a.k2 = k2; a.k3 = k3; a.y = y; a.phi1 = phi1; a.phi2 = phi2; a.rho = rho;
   a.rhs2 = rhs2; a.cr = cr; a.cz = cz; a.cp = cp; a.cq = cq; a.b2 = b2; a.hout = hout; a.err = err;
   return a;
@@ -725,12 +927,24 @@ void apply_budget(nmg_batch *b) {
 
 size_t smem_bytes(const nmg_batch *b) { return sizeof(float) * (size_t)b->ld_max; }
 
-int launch_run(nmg_batch *b) {
-  nmg::BatchArgs a = b->args();
-  cudaMemsetAsync(b->queue.p, 0, sizeof(int), b->stream);
-  nmg::k_batch_run<<<b->blocks, b->threads, smem_bytes(b), b->stream>>>(a);
-  return cudaGetLastError() == cudaSuccess ? 0 : 100;
+// A launch of b->blocks CTAs, in clusters of kTeam where the batch has team particles.
+template <class... Args>
+int launch_batch(nmg_batch *b, void (*kernel)(Args...), Args... args) {
+  cudaMemsetAsync(b->queue.p, 0, 2 * sizeof(int), b->stream);
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(b->blocks);
+  c.blockDim = dim3(b->threads);
+  c.dynamicSmemBytes = smem_bytes(b);
+  c.stream = b->stream;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = b->n_team > 0 ? nmg::kTeam : 1;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, args...) == cudaSuccess ? 0 : 100;
 }
+int launch_run(nmg_batch *b) { return launch_batch(b, nmg::k_batch_run, b->args()); }
 
 int sync_check(nmg_batch *b, const char *where) {
   cudaError_t e = cudaStreamSynchronize(b->stream);
@@ -764,7 +978,11 @@ int set_threads(nmg_batch *b, int threads) {
   }
   cudaFuncSetAttribute(nmg::k_batch_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(b));
   b->threads = threads;
-  b->blocks = std::min(b->P, per * b->sm_count);
+  b->n_team = threads == nmg::kTeamThreads ? b->n_large : 0;   // a team reproduces the sums of that CTA
+  // every resident CTA, but no more than have a particle to work on
+  const int small = b->P - b->n_team;
+  b->blocks = std::min(std::max(small, nmg::kTeam * b->n_team), per * b->sm_count);
+  if (b->n_team > 0) b->blocks = std::max(1, b->blocks / nmg::kTeam) * nmg::kTeam;
   drop_graph(b);
   return 0;
 }
@@ -895,6 +1113,9 @@ int nmg_batch_create(const nmg_particle *parts, int n, const nmg_batch_options *
       v.insert(v.end(), hs[p].D.begin() + c * z, hs[p].D.begin() + (c + 1) * z);
     });
   }
+  up64(b->dinv, on, [&](int p, std::vector<double> &v) {
+    for (int32_t q : hs[p].dg) v.push_back(1.0 / hs[p].K[q]);
+  });
   up64(b->vol, on, [&](int p, std::vector<double> &v) { v.insert(v.end(), hs[p].vol.begin(), hs[p].vol.end()); });
   {
     std::vector<float> all;
@@ -916,11 +1137,21 @@ int nmg_batch_create(const nmg_particle *parts, int n, const nmg_batch_options *
     if (v->alloc(on) || cudaMemset(v->p, 0, sizeof(double) * on)) rc = 100;
   if (b->b2.alloc(std::max<long long>(onb, 1))) rc = 100;
   if (b->err.alloc(1) || cudaMemset(b->err.p, 0, sizeof(int))) rc = 100;
-  if (b->queue.alloc(1)) rc = 100;
-  // queue order: decreasing cost
+  if (b->queue.alloc(2)) rc = 100;
+  // Particles for teams: those one CTA would still be working on when the SMs
+  // had shared the rest evenly (the ROS2 integrator is one CTA's work).
+  std::vector<char> team(n, 0);
+  double all = 0.0;
+  for (const nmg::PDesc &d : b->hdesc) all += d.cost;
+  for (int p = 0; p < n; ++p)
+    team[p] = opt->integrator == 0 && b->hdesc[p].N >= 2 * nmg::kTeamThreads && b->hdesc[p].cost > all / b->sm_count;
+  // queue order: team particles, then the others, each by decreasing cost
   std::vector<int32_t> ord(n);
   std::iota(ord.begin(), ord.end(), 0);
-  std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return b->hdesc[x].cost > b->hdesc[y].cost; });
+  std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) {
+    return team[x] != team[y] ? team[x] > team[y] : b->hdesc[x].cost > b->hdesc[y].cost;
+  });
+  b->n_large = (int)std::count(team.begin(), team.end(), 1);
   if (b->order.alloc(n) || cudaMemcpy(b->order.p, ord.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice)) rc = 100;
   // per-particle state
   std::vector<nmg::PState> st(n);
@@ -996,9 +1227,7 @@ int nmg_batch_get_m(const nmg_batch *b, double *m) {
 int nmg_batch_eval(nmg_batch *b, double *dmdt, double *h_total) {
   if (!b) return -1;
   nmg::BatchArgs a = b->args();
-  cudaMemsetAsync(b->queue.p, 0, sizeof(int), b->stream);
-  nmg::k_batch_eval<<<b->blocks, b->threads, smem_bytes(b), b->stream>>>(a, b->dmdt);
-  if (cudaGetLastError() != cudaSuccess) return bfail(b, 100, "nmg_batch_eval: launch failed");
+  if (launch_batch(b, nmg::k_batch_eval, a, b->dmdt.p)) return bfail(b, 100, "nmg_batch_eval: launch failed");
   int rc = sync_check(b, "nmg_batch_eval");
   if (rc) return rc;
   if (dmdt) cudaMemcpy(dmdt, b->dmdt.p, sizeof(double) * 3 * b->Ntot, cudaMemcpyDeviceToHost);
@@ -1016,8 +1245,10 @@ int nmg_batch_run(nmg_batch *b, int launches) {
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
       return bfail(b, 100, "nmg_batch_run: capture failed");
-    for (int k = 0; k < launches; ++k) launch_run(b);
-    if (cudaStreamEndCapture(b->stream, &g) != cudaSuccess || !g) {
+    int bad = 0;
+    for (int k = 0; k < launches; ++k) bad |= launch_run(b);
+    if (cudaStreamEndCapture(b->stream, &g) != cudaSuccess || !g || bad) {
+      if (g) cudaGraphDestroy(g);
       cudaGetLastError();
       return bfail(b, 100, "nmg_batch_run: capture failed");
     }
