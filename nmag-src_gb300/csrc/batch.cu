@@ -1038,7 +1038,7 @@ int nmg_batch_create(const nmg_particle *parts, int n, const nmg_batch_options *
     if (!rc) rc = nmg::build_mesh(h, q.coords, q.tets, err);
     if (!rc) {
       h->mesh.ld = (h->mesh.nb + 7) / 8 * 8;
-      rc = nmg::fill_bem(h, err);
+      rc = nmg::fill_bem(h, err, true);
     }
     if (rc) {
       h->stream = nullptr;

@@ -5,19 +5,37 @@
 // (src/bem3d_stubs.c:413-610) for every (surface triangle, observer row), then
 // adding Omega_i/(4 pi) - 1 on the diagonal (bem3d.ml:1040-1043).
 //
-// Layout: the fill accumulates into a column-major buffer, a[c*nb + k] =
-// B[k][c] (k = observer row, c = boundary column).  One thread owns one
-// observer row and walks the triangles in the reference's order, so every
-// entry is accumulated in exactly the reference's order with no atomics, and a
-// warp's 32 rows are adjacent in memory (coalesced read-modify-write).  A tiled
+// The formula's parts that neighbouring triangles share are formed once: for a
+// chunk of observers the distances to the boundary nodes, the logarithms of
+// the surface edges, and every triangle's solid angle and distance from its
+// plane; then one thread per (column, observer) adds the column's triangles in
+// the reference's order, so every entry is accumulated in exactly that order
+// with no atomics and written once.  A warp holds 32 observers of one node,
+// edge, triangle or column, so geometry loads are uniform and every other
+// access is coalesced.  The chunk is as large as keeps its arrays (8 bytes per
+// observer and node, edge, and twice per triangle) in L2.
+//
+// Bound by the FP64 pipe: ~165 operations a pair, against ~350 with three
+// logarithms, an arc cosine and three distances per triangle and one thread
+// per observer row (which left the chip half idle below ~20,000 rows).  8,562
+// x 17,120 pairs: 245 ms before, 30 now (angles 51 %, edges 27 %, columns 16 %,
+// distances 6 %); the film's 8.8e8: a handle in 1,086 ms before, 280 now; the
+// 30 nm cube's in 23, 2.4 now.  The expressions the angle's rounding depends on
+// (it is the arc cosine of a number near 1) follow the reference's operation
+// order; this file is compiled with --fmad=false, and fma() is written where it
+// is wanted.
+//
+// The columns leave as a[c*nb + k] = B[k][c] (k = observer row); a tiled
 // transpose then stores the matrix row-major with the row stride padded to a
 // multiple of 8 (bem[k*ld + c]), the layout the matrix-vector product streams.
-// Compiled with --fmad=false to follow the written operation order.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <numeric>
+#include <vector>
 
 #include "nmg_internal.h"
 
@@ -80,68 +98,174 @@ __global__ void k_tri_setup(int ntri, const int32_t *__restrict__ tri, const dou
 // Running maximum of |observer coordinate| in row order: the reference's
 // geo_eps = 1e-13 * max over the triangle and the observers visited so far
 // within one block call (bem3d_stubs.c:531-533).
-__global__ void k_observer_prefix_max(int nb, const int32_t *__restrict__ node_of_b, const double *__restrict__ X,
-                                      double *__restrict__ out) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+// One block: tiles of its threads, a shuffle scan in each.
+__global__ void __launch_bounds__(1024) k_observer_prefix_max(int nb, const int32_t *__restrict__ node_of_b,
+                                                              const double *__restrict__ X,
+                                                              double *__restrict__ out) {
+  __shared__ double wmax[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double run = 0.0;
-  for (int k = 0; k < nb; ++k) {
-    const double *o = X + 3 * (size_t)node_of_b[k];
-    for (int d = 0; d < 3; ++d) { double a = fabs(o[d]); if (a > run) run = a; }
-    out[k] = run;
+  for (int base = 0; base < nb; base += blockDim.x) {
+    const int k = base + threadIdx.x;
+    double a = 0.0;
+    if (k < nb) {
+      const double *o = X + 3 * (size_t)node_of_b[k];
+      for (int d = 0; d < 3; ++d) { const double v = fabs(o[d]); if (v > a) a = v; }
+    }
+    for (int s = 1; s < 32; s <<= 1) {
+      const double v = __shfl_up_sync(0xffffffffu, a, s);
+      if (lane >= s && v > a) a = v;
+    }
+    if (lane == 31) wmax[w] = a;
+    __syncthreads();
+    for (int q = 0; q < w; ++q) if (wmax[q] > a) a = wmax[q];
+    if (run > a) a = run;
+    if (k < nb) out[k] = a;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) if (wmax[q] > run) run = wmax[q];
+    __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(128) k_bem_fill(int nb, int ntri, const TriGeo *__restrict__ geo,
-                                                  const int32_t *__restrict__ tri,
-                                                  const int32_t *__restrict__ node_of_b,
-                                                  const double *__restrict__ X, const double *__restrict__ obs_max,
-                                                  const double *__restrict__ solid_angle, double *__restrict__ bem) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nb) return;
-  const double ox = X[3 * (size_t)node_of_b[k]], oy = X[3 * (size_t)node_of_b[k] + 1],
-               oz = X[3 * (size_t)node_of_b[k] + 2];
-  const double omax = obs_max[k];
-  for (int t = 0; t < ntri; ++t) {
-    const TriGeo &g = geo[t];
-    if (!g.ok) continue;
-    double r[3][3], rl[3];
-    for (int v = 0; v < 3; ++v) {
-      r[v][0] = g.p[v][0] - ox; r[v][1] = g.p[v][1] - oy; r[v][2] = g.p[v][2] - oz;
-      rl[v] = sqrt(r[v][0] * r[v][0] + r[v][1] * r[v][1] + r[v][2] * r[v][2]);
-    }
-    if (rl[0] <= 0.0 || rl[1] <= 0.0 || rl[2] <= 0.0) continue;
-    double vlog0 = log((rl[1] + rl[2] + g.s_l[0]) / (rl[1] + rl[2] - g.s_l[0]));
-    double vlog1 = log((rl[2] + rl[0] + g.s_l[1]) / (rl[2] + rl[0] - g.s_l[1]));
-    double vlog2 = log((rl[0] + rl[1] + g.s_l[2]) / (rl[0] + rl[1] - g.s_l[2]));
-    double sp01 = r[0][0] * r[1][0] + r[0][1] * r[1][1] + r[0][2] * r[1][2];
-    double sp12 = r[1][0] * r[2][0] + r[1][1] * r[2][1] + r[1][2] * r[2][2];
-    double sp20 = r[2][0] * r[0][0] + r[2][1] * r[0][1] + r[2][2] * r[0][2];
-    double num = rl[0] * rl[1] * rl[2] + rl[0] * sp12 + rl[1] * sp20 + rl[2] * sp01;
-    double den = sqrt(2.0 * (rl[1] * rl[2] + sp12) * (rl[2] * rl[0] + sp20) * (rl[0] * rl[1] + sp01));
-    if (den == 0.0) continue;
-    double angle = num / den;
-    angle = angle < -1.0 ? -1.0 : (angle > 1.0 ? 1.0 : angle);
-    angle = 2.0 * acos(angle);
-    double zeta = g.zeta_v[0] * r[0][0] + g.zeta_v[1] * r[0][1] + g.zeta_v[2] * r[0][2];
-    if (zeta < 0.0) angle = -angle;
-    double f = g.factor;
-    double geo_eps = (g.maxgeo > omax ? g.maxgeo : omax) * 1e-13;
-    if (fabs(zeta) < geo_eps) f = 0.0;
-    double gl0 = 1.0 * vlog0 + g.gam01 * vlog1 + g.gam20 * vlog2;
-    double gl1 = g.gam01 * vlog0 + 1.0 * vlog1 + g.gam12 * vlog2;
-    double gl2 = g.gam20 * vlog0 + g.gam12 * vlog1 + 1.0 * vlog2;
-    double e0 = g.eta[0][0] * r[1][0] + g.eta[0][1] * r[1][1] + g.eta[0][2] * r[1][2];
-    double e1 = g.eta[1][0] * r[2][0] + g.eta[1][1] * r[2][1] + g.eta[1][2] * r[2][2];
-    double e2 = g.eta[2][0] * r[0][0] + g.eta[2][1] * r[0][1] + g.eta[2][2] * r[0][2];
-    double lh0 = f * g.s_l[0] * (angle * e0 - zeta * gl0);
-    double lh1 = f * g.s_l[1] * (angle * e1 - zeta * gl1);
-    double lh2 = f * g.s_l[2] * (angle * e2 - zeta * gl2);
-    const int32_t *tv = tri + 3 * (size_t)t;
-    bem[(size_t)tv[0] * nb + k] += lh0;
-    bem[(size_t)tv[1] * nb + k] += lh1;
-    bem[(size_t)tv[2] * nb + k] += lh2;
+// What the sums need of a triangle's vertex v: eta_v and eta_v . p_(v+1), f s_v,
+// and the direction cosines between edge v and the two after it.
+struct VertexGeo {
+  double eta[3], etap, fs, ga, gb;
+};
+__global__ void k_vertex_geo(int ntri, const TriGeo *__restrict__ geo, VertexGeo *__restrict__ out) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 3 * ntri) return;
+  const TriGeo &g = geo[e / 3];
+  const int v = e % 3, n = v == 2 ? 0 : v + 1;
+  VertexGeo o;
+  for (int d = 0; d < 3; ++d) o.eta[d] = g.eta[v][d];
+  o.etap = g.eta[v][0] * g.p[n][0] + g.eta[v][1] * g.p[n][1] + g.eta[v][2] * g.p[n][2];
+  o.fs = g.factor * g.s_l[v];
+  o.ga = v == 0 ? g.gam01 : (v == 1 ? g.gam12 : g.gam20);   // edges v, v + 1
+  o.gb = v == 0 ? g.gam20 : (v == 1 ? g.gam01 : g.gam12);   // edges v, v + 2
+  out[e] = o;
+}
+
+// The observers [k0, k0 + kc) of a chunk; arrays are [item][kc].
+struct FillArgs {
+  int nb, ne, ntri, k0, kc;
+  const int32_t *node_of_b, *tri, *edge, *tri_edge, *col_ptr, *col_tri;   // col_tri: 3 triangle + vertex, ascending
+  const double *X, *edge_len, *obs_max, *solid_angle;
+  const TriGeo *geo;
+  const VertexGeo *vgeo;
+  double *dist, *lg, *ang, *zeta, *bem;
+};
+
+// Distance of every boundary node from every observer of the chunk.
+__global__ void __launch_bounds__(256) k_fill_dist(FillArgs a) {
+  const int k = blockIdx.x * 32 + (threadIdx.x & 31), v = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (k >= a.kc || v >= a.nb || a.k0 + k >= a.nb) return;
+  const double *o = a.X + 3 * (size_t)a.node_of_b[a.k0 + k], *p = a.X + 3 * (size_t)a.node_of_b[v];
+  const double r0 = p[0] - o[0], r1 = p[1] - o[1], r2 = p[2] - o[2];
+  a.dist[(size_t)v * a.kc + k] = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
+}
+
+// kExact in the next three: every entry as the reference's operation order
+// rounds it, for matrices that are then rounded to 24 bits (the particle batch,
+// whose adaptive steps one entry rounded the other way moves by 1e-6; the FP32
+// and the split-BF16 forms, whose products it moves by 1e-7 in its row).
+
+// log((a + b + s) / (a + b - s)) of every surface edge (length s, its ends at
+// distances a and b): 2 artanh(s / (a + b)), by its series where the edge is
+// far (the truncation is below 2^-58), by the logarithm where it is near.
+template <bool kExact>
+__global__ void __launch_bounds__(256) k_fill_edges(FillArgs a) {
+  const int k = blockIdx.x * 32 + (threadIdx.x & 31), e = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (k >= a.kc || e >= a.ne || a.k0 + k >= a.nb) return;
+  const double L = a.dist[(size_t)a.edge[2 * e] * a.kc + k] + a.dist[(size_t)a.edge[2 * e + 1] * a.kc + k];
+  const double s = a.edge_len[e];
+  double v;
+  if (!kExact && 8.0 * s <= L) {
+    const double x = s / L, y = x * x;
+    double t = 1.0 / 17.0;
+    t = fma(t, y, 1.0 / 15.0); t = fma(t, y, 1.0 / 13.0); t = fma(t, y, 1.0 / 11.0); t = fma(t, y, 1.0 / 9.0);
+    t = fma(t, y, 1.0 / 7.0);  t = fma(t, y, 1.0 / 5.0);  t = fma(t, y, 1.0 / 3.0);
+    v = 2.0 * fma(x * y, t, x);
+  } else {
+    v = log((L + s) / (L - s));
   }
-  bem[(size_t)k * nb + k] += solid_angle[k] / (4.0 * kPi) - 1.0;
+  a.lg[(size_t)e * a.kc + k] = v;
+}
+
+// Signed solid angle and distance from the plane of every triangle; angle NaN:
+// the triangle adds nothing (degenerate, the observer one of its vertices or
+// in its plane, bem3d_stubs.c:531-600).
+template <bool kExact>
+__global__ void __launch_bounds__(256) k_fill_angles(FillArgs a) {
+  const int k = blockIdx.x * 32 + (threadIdx.x & 31), t = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (k >= a.kc || t >= a.ntri || a.k0 + k >= a.nb) return;
+  const TriGeo &g = a.geo[t];
+  const int32_t *tv = a.tri + 3 * (size_t)t;
+  const double *o = a.X + 3 * (size_t)a.node_of_b[a.k0 + k];
+  const double ox = o[0], oy = o[1], oz = o[2], omax = a.obs_max[a.k0 + k];
+  double r[3][3], rl[3];
+  for (int v = 0; v < 3; ++v) {
+    r[v][0] = g.p[v][0] - ox; r[v][1] = g.p[v][1] - oy; r[v][2] = g.p[v][2] - oz;
+    rl[v] = a.dist[(size_t)tv[v] * a.kc + k];
+  }
+  double angle = nan("");
+  const double zeta = g.zeta_v[0] * r[0][0] + g.zeta_v[1] * r[0][1] + g.zeta_v[2] * r[0][2];
+  const double geo_eps = (g.maxgeo > omax ? g.maxgeo : omax) * 1e-13;
+  if (g.ok && rl[0] > 0.0 && rl[1] > 0.0 && rl[2] > 0.0 && !(fabs(zeta) < geo_eps)) {
+    const double sp01 = r[0][0] * r[1][0] + r[0][1] * r[1][1] + r[0][2] * r[1][2];
+    const double sp12 = r[1][0] * r[2][0] + r[1][1] * r[2][1] + r[1][2] * r[2][2];
+    const double sp20 = r[2][0] * r[0][0] + r[2][1] * r[0][1] + r[2][2] * r[0][2];
+    const double num = rl[0] * rl[1] * rl[2] + rl[0] * sp12 + rl[1] * sp20 + rl[2] * sp01;
+    const double den = sqrt(2.0 * (rl[1] * rl[2] + sp12) * (rl[2] * rl[0] + sp20) * (rl[0] * rl[1] + sp01));
+    if (den != 0.0) {
+      double q = num / den;
+      q = q < -1.0 ? -1.0 : (q > 1.0 ? 1.0 : q);
+      const double y = 0.5 * (1.0 - q);   // exact for q >= 1/2
+      if (!kExact && y < 0.0078125) {   // acos q = 2 asin sqrt y, the arc sine's series (truncation below 2^-58)
+        double p = 143.0 / 10240.0;
+        p = fma(p, y, 231.0 / 13312.0); p = fma(p, y, 63.0 / 2816.0); p = fma(p, y, 35.0 / 1152.0);
+        p = fma(p, y, 5.0 / 112.0);     p = fma(p, y, 3.0 / 40.0);    p = fma(p, y, 1.0 / 6.0);
+        const double s = sqrt(y);
+        angle = 4.0 * fma(s * y, p, s);
+      } else {
+        angle = 2.0 * acos(q);
+      }
+      if (zeta < 0.0) angle = -angle;
+    }
+  }
+  a.ang[(size_t)t * a.kc + k] = angle;
+  a.zeta[(size_t)t * a.kc + k] = zeta;
+}
+
+// Entry (observer, column): the column's triangles in order.
+template <bool kExact>
+__global__ void __launch_bounds__(256) k_fill_columns(FillArgs a) {
+  const int k = blockIdx.x * 32 + (threadIdx.x & 31), c = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (k >= a.kc || c >= a.nb || a.k0 + k >= a.nb) return;
+  const double *o = a.X + 3 * (size_t)a.node_of_b[a.k0 + k];
+  const double ox = o[0], oy = o[1], oz = o[2];
+  double acc = 0.0;
+  for (int q = a.col_ptr[c]; q < a.col_ptr[c + 1]; ++q) {
+    const int e = a.col_tri[q], t = e / 3, v = e - 3 * t, n = v == 2 ? 0 : v + 1, m = n == 2 ? 0 : n + 1;
+    const double angle = a.ang[(size_t)t * a.kc + k], zeta = a.zeta[(size_t)t * a.kc + k];
+    if (angle != angle) continue;
+    const VertexGeo &g = a.vgeo[e];
+    const int32_t *te = a.tri_edge + 3 * (size_t)t;
+    const double lv = a.lg[(size_t)te[v] * a.kc + k], ln = a.lg[(size_t)te[n] * a.kc + k],
+                 lm = a.lg[(size_t)te[m] * a.kc + k];
+    if (kExact) {   // the three products of a row of the direction cosines in the reference's order
+      const double *p = a.X + 3 * (size_t)a.node_of_b[a.tri[3 * (size_t)t + n]];
+      const double r0 = p[0] - ox, r1 = p[1] - oy, r2 = p[2] - oz;
+      const double e0 = g.eta[0] * r0 + g.eta[1] * r1 + g.eta[2] * r2;
+      const double gl = v == 0 ? lv + g.ga * ln + g.gb * lm : (v == 1 ? g.gb * lm + lv + g.ga * ln : g.ga * ln + g.gb * lm + lv);
+      acc += g.fs * (angle * e0 - zeta * gl);
+      continue;
+    }
+    const double gl = fma(g.gb, lm, fma(g.ga, ln, lv));
+    const double en = fma(-g.eta[2], oz, fma(-g.eta[1], oy, fma(-g.eta[0], ox, g.etap)));
+    acc = fma(g.fs, fma(angle, en, -(zeta * gl)), acc);
+  }
+  if (c == a.k0 + k) acc += a.solid_angle[c] / (4.0 * kPi) - 1.0;
+  a.bem[(size_t)c * a.nb + a.k0 + k] = acc;
 }
 
 // Column-major fill buffer (a[c*nb + k]) -> row-major matrix with padded row
@@ -220,10 +344,11 @@ __global__ void k_pack_bem16f(int nb, int ld, int KT, long long ntiles, const fl
 
 }  // namespace
 
-int fill_bem(nmg_handle *h, std::string &err) {
+int fill_bem(nmg_handle *h, std::string &err, bool exact) {
   Mesh &M = h->mesh;
   cudaStream_t s = h->stream;
   if (M.nb == 0) return 0;
+  exact = exact || h->opt.bem_precision == 1 || h->opt.bem_precision == 3;
   const size_t nb = M.nb;
   if (M.ld != (M.nb + 7) / 8 * 8) {
     err = "BEM row stride not set up by the workspace";
@@ -236,11 +361,83 @@ int fill_bem(nmg_handle *h, std::string &err) {
     // temporary; one tiled transpose then gives the row-major product layout.
     DevBuf<double> colmajor;
     NMG_CUDA_TRY(colmajor.alloc(nb * nb), "alloc BEM fill buffer (nb^2 doubles)");
-    NMG_CUDA_TRY(cudaMemsetAsync(colmajor.p, 0, sizeof(double) * nb * nb, s), "zero BEM");
     k_tri_setup<<<(M.ntri + 127) / 128, 128, 0, s>>>(M.ntri, M.tri, M.tri_normal, M.node_of_b, M.coords, M.trigeo);
-    k_observer_prefix_max<<<1, 32, 0, s>>>(M.nb, M.node_of_b, M.coords, M.obs_max);
-    k_bem_fill<<<(M.nb + 127) / 128, 128, 0, s>>>(M.nb, M.ntri, M.trigeo, M.tri, M.node_of_b, M.coords, M.obs_max,
-                                                   M.solid_angle, colmajor);
+    k_observer_prefix_max<<<1, 1024, 0, s>>>(M.nb, M.node_of_b, M.coords, M.obs_max);
+    // the surface's edges and every column's triangles
+    const int nt = M.ntri;
+    std::vector<int32_t> tri(3 * (size_t)nt);
+    std::vector<TriGeo> geo(nt);
+    NMG_CUDA_TRY(cudaMemcpyAsync(tri.data(), M.tri.p, sizeof(int32_t) * tri.size(), cudaMemcpyDeviceToHost, s), "d2h");
+    NMG_CUDA_TRY(cudaMemcpyAsync(geo.data(), M.trigeo.p, sizeof(TriGeo) * nt, cudaMemcpyDeviceToHost, s), "d2h");
+    NMG_CUDA_TRY(cudaStreamSynchronize(s), "surface triangles");
+    std::vector<std::pair<uint64_t, int32_t>> key(3 * (size_t)nt);
+    for (int t = 0; t < nt; ++t)
+      for (int v = 0; v < 3; ++v) {   // edge v faces vertex v
+        const uint64_t x = tri[3 * (size_t)t + (v + 1) % 3], y = tri[3 * (size_t)t + (v + 2) % 3];
+        key[3 * (size_t)t + v] = {std::min(x, y) << 32 | std::max(x, y), 3 * t + v};
+      }
+    std::sort(key.begin(), key.end());
+    std::vector<int32_t> edge, tri_edge(3 * (size_t)nt), col_ptr(nb + 1, 0), col_tri(3 * (size_t)nt);
+    std::vector<double> edge_len;
+    for (size_t q = 0; q < key.size(); ++q) {
+      if (q == 0 || key[q].first != key[q - 1].first) {
+        edge.push_back((int32_t)(key[q].first >> 32));
+        edge.push_back((int32_t)(key[q].first & 0xffffffffu));
+        edge_len.push_back(geo[key[q].second / 3].s_l[key[q].second % 3]);   // the same from either side, bit for bit
+      }
+      tri_edge[key[q].second] = (int32_t)edge_len.size() - 1;
+    }
+    for (int32_t c : tri) ++col_ptr[c + 1];
+    std::partial_sum(col_ptr.begin(), col_ptr.end(), col_ptr.begin());
+    {
+      std::vector<int32_t> at(col_ptr.begin(), col_ptr.end() - 1);
+      for (int32_t e = 0; e < 3 * nt; ++e) col_tri[at[tri[e]]++] = e;
+    }
+    const int ne = (int)edge_len.size();
+    const size_t per = nb + ne + 2 * (size_t)nt;   // doubles per observer of a chunk
+    int kc = (int)std::min<size_t>((nb + 31) / 32 * 32, std::max<size_t>(32, (72u << 20) / (8 * per) / 32 * 32));
+    DevBuf<int32_t> dedge, dte, dcp, dct;
+    DevBuf<double> dlen, work;
+    DevBuf<VertexGeo> vg;
+    NMG_CUDA_TRY(dedge.alloc(std::max<size_t>(edge.size(), 1)), "alloc");
+    NMG_CUDA_TRY(dte.alloc(std::max<size_t>(tri_edge.size(), 1)), "alloc");
+    NMG_CUDA_TRY(dcp.alloc(nb + 1), "alloc");
+    NMG_CUDA_TRY(dct.alloc(std::max<size_t>(col_tri.size(), 1)), "alloc");
+    NMG_CUDA_TRY(dlen.alloc(std::max(ne, 1)), "alloc");
+    NMG_CUDA_TRY(vg.alloc(std::max(3 * (size_t)nt, (size_t)1)), "alloc");
+    NMG_CUDA_TRY(work.alloc(per * kc), "alloc BEM fill chunk");
+    NMG_CUDA_TRY(cudaMemcpyAsync(dedge.p, edge.data(), sizeof(int32_t) * edge.size(), cudaMemcpyHostToDevice, s), "h2d");
+    NMG_CUDA_TRY(cudaMemcpyAsync(dte.p, tri_edge.data(), sizeof(int32_t) * tri_edge.size(), cudaMemcpyHostToDevice, s), "h2d");
+    NMG_CUDA_TRY(cudaMemcpyAsync(dcp.p, col_ptr.data(), sizeof(int32_t) * (nb + 1), cudaMemcpyHostToDevice, s), "h2d");
+    NMG_CUDA_TRY(cudaMemcpyAsync(dct.p, col_tri.data(), sizeof(int32_t) * col_tri.size(), cudaMemcpyHostToDevice, s), "h2d");
+    NMG_CUDA_TRY(cudaMemcpyAsync(dlen.p, edge_len.data(), sizeof(double) * ne, cudaMemcpyHostToDevice, s), "h2d");
+    if (nt > 0) k_vertex_geo<<<(3 * nt + 127) / 128, 128, 0, s>>>(nt, M.trigeo, vg);
+    FillArgs a;
+    a.nb = M.nb; a.ne = ne; a.ntri = nt; a.kc = kc;
+    a.node_of_b = M.node_of_b; a.tri = M.tri; a.edge = dedge; a.tri_edge = dte; a.col_ptr = dcp; a.col_tri = dct;
+    a.X = M.coords; a.edge_len = dlen; a.obs_max = M.obs_max; a.solid_angle = M.solid_angle;
+    a.geo = M.trigeo; a.vgeo = vg;
+    a.dist = work; a.lg = a.dist + nb * kc; a.ang = a.lg + (size_t)ne * kc; a.zeta = a.ang + (size_t)nt * kc;
+    a.bem = colmajor;
+    // grid.y ends at 65,535: eight items a block
+    if ((std::max<size_t>(std::max<size_t>(nb, ne), nt) + 7) / 8 > 65535) {
+      err = "BEM fill: surface too large (more than 524,280 nodes, edges or triangles)";
+      return 3;
+    }
+    for (a.k0 = 0; a.k0 < M.nb; a.k0 += kc) {
+      const unsigned gx = (unsigned)((std::min(kc, M.nb - a.k0) + 31) / 32);
+      k_fill_dist<<<dim3(gx, (M.nb + 7) / 8), 256, 0, s>>>(a);
+      const dim3 ge(gx, (ne + 7) / 8), gt(gx, (nt + 7) / 8), gc(gx, (M.nb + 7) / 8);
+      if (exact) {
+        if (ne > 0) k_fill_edges<true><<<ge, 256, 0, s>>>(a);
+        if (nt > 0) k_fill_angles<true><<<gt, 256, 0, s>>>(a);
+        k_fill_columns<true><<<gc, 256, 0, s>>>(a);
+      } else {
+        if (ne > 0) k_fill_edges<false><<<ge, 256, 0, s>>>(a);
+        if (nt > 0) k_fill_angles<false><<<gt, 256, 0, s>>>(a);
+        k_fill_columns<false><<<gc, 256, 0, s>>>(a);
+      }
+    }
     NMG_CUDA_TRY(cudaGetLastError(), "bem fill launch");
     NMG_CUDA_TRY(M.bem.alloc(nb * M.ld), "alloc BEM (nb x ld doubles)");
     dim3 tb(32, 8), tg((M.ld + 31) / 32, (M.nb + 31) / 32);

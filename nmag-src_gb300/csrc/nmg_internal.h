@@ -352,7 +352,8 @@ int build_mesh(nmg_handle *h, const double *coords, const int32_t *tets, std::st
 int export_operator(const nmg_handle *h, int which, double coeff, int *rows, int *cols, int *nnz,
                     int32_t *rp, int32_t *ci, double *vals);
 // ---- bem_kernels.cu ----
-int fill_bem(nmg_handle *h, std::string &err);
+// exact: entries rounded as the reference's operation order rounds them (for FP32 copies)
+int fill_bem(nmg_handle *h, std::string &err, bool exact = false);
 void bem_gemv(nmg_handle *h, const double *x, double *y);
 // ---- nmg_sites.cu (several materials) ----
 int rhs_eval_sites(nmg_handle *h, const double *d_m, double *d_dmdt);
