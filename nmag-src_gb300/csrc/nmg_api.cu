@@ -417,11 +417,10 @@ int nmg_bem_apply(nmg_handle *h, const double *d_x, double *d_y, int n_rhs) {
   if (n_rhs < 1) return fail(h, -2, "nmg_bem_apply: n_rhs must be positive");
   if (h->mesh.nb == 0) return fail(h, -2, "nmg_bem_apply: the mesh has no boundary");
   if (h->anchored()) return fail(h, -2, "nmg_bem_apply: not available with the anchored product (bem_anchor_tol)");
-  const size_t nb = h->mesh.nb;
   if (h->opt.bem_precision == 3) {
     if (nmg::bem_tc(h, d_x, d_y, n_rhs)) return fail(h, 100, "nmg_bem_apply: " + h->last_error);
   } else {
-    for (int n = 0; n < n_rhs; ++n) nmg::bem_gemv(h, d_x + n * nb, d_y + n * nb);
+    nmg::bem_apply(h, d_x, d_y, n_rhs);
   }
   if (cudaGetLastError() != cudaSuccess) return fail(h, 100, "nmg_bem_apply: launch failed");
   return nmg::check_device_error(h, "nmg_bem_apply");

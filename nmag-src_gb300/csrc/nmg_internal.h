@@ -128,6 +128,7 @@ struct Workspace {
   DevBuf<unsigned long long> anc_mx;
   DevBuf<int> anc_flag;
   DevBuf<long long> anc_count;
+  DevBuf<double> apply_part;   // nmg_bem_apply's passes: partials and x pairs (allocated on first use)
   // m at the last nmg_max_dm_step / nmg_set_m (allocated on first use)
   DevBuf<double> m_mark;
   // FP16 fragment product: x - x0 of 8 members in B-fragment order, the
@@ -355,6 +356,7 @@ int export_operator(const nmg_handle *h, int which, double coeff, int *rows, int
 // exact: entries rounded as the reference's operation order rounds them (for FP32 copies)
 int fill_bem(nmg_handle *h, std::string &err, bool exact = false);
 void bem_gemv(nmg_handle *h, const double *x, double *y);
+void bem_apply(nmg_handle *h, const double *x, double *y, int n);   // n vectors, not the tensor-core form
 // ---- nmg_sites.cu (several materials) ----
 int rhs_eval_sites(nmg_handle *h, const double *d_m, double *d_dmdt);
 int energy_density_sites(nmg_handle *h, const double *d_m, double *d_E5);

@@ -1594,7 +1594,8 @@ __global__ void k_to_f32_vec(int n, int ld, const double *__restrict__ a, float 
 // k_gemv_*, every matrix unit multiplied into all members' accumulators, so
 // the matrix is streamed once per nm right-hand sides.  Partials at
 // part[(w * maxr + row slot) * MB + m].
-template <int MB>
+// kFull: nm == MB, so that no member's loads wait on a comparison with nm.
+template <int MB, bool kFull>
 __global__ void __launch_bounds__(kGemvThreads) k_gemm_f64(int nb, int ld, long long seg, int maxr, int nm,
                                                             const double *__restrict__ B,
                                                             const double *__restrict__ x, double *__restrict__ part) {
@@ -1610,6 +1611,7 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemm_f64(int nb, int ld, long 
     double acc[MB];
 #pragma unroll
     for (int m = 0; m < MB; ++m) acc[m] = 0.0;
+#pragma unroll 2
     for (long long q = a + lane; q < e; q += 32) {
       const double2 *p = reinterpret_cast<const double2 *>(row + 4 * (q - r * Q));
       const double2 v0 = __ldcs(p), v1 = __ldcs(p + 1);
@@ -1617,7 +1619,7 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemm_f64(int nb, int ld, long 
       const int c0 = min(c, nb - 1), c1 = min(c + 1, nb - 1), c2 = min(c + 2, nb - 1), c3 = min(c + 3, nb - 1);
 #pragma unroll
       for (int m = 0; m < MB; ++m) {
-        if (m >= nm) break;
+        if (!kFull && m >= nm) break;
         const double *xm = x + (size_t)m * nb;
         double t = fma(v0.x, __ldg(xm + c0), acc[m]);
         t = fma(v0.y, __ldg(xm + c1), t);
@@ -1627,7 +1629,7 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemm_f64(int nb, int ld, long 
     }
 #pragma unroll
     for (int m = 0; m < MB; ++m) {
-      if (m >= nm) break;
+      if (!kFull && m >= nm) break;
       const double s = warp_sum(acc[m]);
       if (lane == 0) part[(w * maxr + (r - rfirst)) * MB + m] = s;
     }
@@ -2875,6 +2877,86 @@ void bem_gemv(nmg_handle *h, const double *x, double *y) {
   ++h->launches;
 }
 
+// One pass of the plain ensemble products (FP64 or compensated): nm <= kChunk
+// vectors, partials (and the compensated form's x pairs behind them) in part.
+static size_t bem_pass_doubles(const nmg_handle *h, size_t *x_off) {
+  const Mesh &M = h->mesh;
+  const Workspace &W = h->ws;
+  size_t n = (size_t)W.gemv_blocks * (kGemvThreads / 32) * W.gemv_maxr[0] * kChunk;
+  n = std::max(n, (size_t)((M.ld + kDfCols - 1) / kDfCols) * M.nb * kChunk);
+  *x_off = (n + 7) / 8 * 8;
+  return *x_off + (size_t)kChunk * M.ld;
+}
+static void bem_pass(nmg_handle *h, const double *x, double *y, int nm, double *part, size_t x_off) {
+  Mesh &M = h->mesh;
+  Workspace &W = h->ws;
+  const int nb = M.nb, MB = nm <= 2 ? 2 : (nm <= 4 ? 4 : 8);
+  if (h->opt.bem_precision == 2 && M.bem16lo.p) {
+    float *xh = reinterpret_cast<float *>(part + x_off), *xl = xh + (size_t)nm * M.ld;
+    k_split_x<<<nblk((long long)M.ld * nm, 256), 256, 0, h->stream>>>(nb, M.ld, nm, x, xh, xl); ++h->launches;
+    const int nslab = (M.ld + kDfCols - 1) / kDfCols;
+    const dim3 grid(nslab, (nb + kDfRows - 1) / kDfRows);
+    NMG_PROF_BEGIN(h, 0);
+    if (MB == 2) k_gemm_df<2><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, M.bem16lo, xh, xl, part);
+    else if (MB == 4) k_gemm_df<4><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, M.bem16lo, xh, xl, part);
+    else k_gemm_df<8><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, M.bem16lo, xh, xl, part);
+    NMG_PROF_END(h);
+    ++h->launches;
+    k_slab_sum_m<<<nblk((long long)nb * nm, 256), 256, 0, h->stream>>>(nb, nslab, nm, MB, part, y); ++h->launches;
+    return;
+  }
+  const long long seg = W.gemv_seg[0];
+  const int maxr = W.gemv_maxr[0];
+  NMG_PROF_BEGIN(h, 0);
+  const dim3 grid(W.gemv_blocks);
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, kGemvThreads, 0, h->stream>>>(nb, M.ld, seg, maxr, nm, M.bem, x, part);
+  };
+  if (nm == MB) {
+    if (MB == 2) launch(k_gemm_f64<2, true>);
+    else if (MB == 4) launch(k_gemm_f64<4, true>);
+    else launch(k_gemm_f64<8, true>);
+  } else {
+    if (MB == 2) launch(k_gemm_f64<2, false>);
+    else if (MB == 4) launch(k_gemm_f64<4, false>);
+    else launch(k_gemm_f64<8, false>);
+  }
+  NMG_PROF_END(h);
+  ++h->launches;
+  k_row_sum_m<<<nblk((long long)nb * nm, 256), 256, 0, h->stream>>>(
+      nb, (long long)(M.ld / 4), seg, maxr, (long long)W.gemv_blocks * (kGemvThreads / 32), nm, MB, part, y);
+  ++h->launches;
+}
+
+// Y = B X for n vectors (vector k at x + k * nb).  The FP64 and compensated
+// forms take up to kChunk vectors per pass over the matrix: the compensated
+// product of one vector streams 6 bytes an entry for 12 FP32 operations (76 us
+// at 8,562 boundary nodes), eight of them share the stream and are bound by
+// the FP32 pipe (271 us); FP64 products are bound by the FP64 pipe either way
+// (8 vectors at 8,562: 1,013 us against 8 x 130; at 602: 30 against 8 x 14) and
+// go in full passes of 8, 4 and 2, whose kernels do not test the count (5
+// vectors in a pass of 8: 803 us, 4 + 1: 640).  The FP32 and tensor-core forms keep their own
+// products (a different order of FP32 sums is a different rounding).
+void bem_apply(nmg_handle *h, const double *x, double *y, int n) {
+  Workspace &W = h->ws;
+  const size_t nb = h->mesh.nb;
+  size_t off = 0;
+  const size_t need = bem_pass_doubles(h, &off);
+  const bool pass = n > 1 && (h->opt.bem_precision == 0 || (h->opt.bem_precision == 2 && h->mesh.bem16lo.p)) &&
+                    (W.apply_part.n >= need || W.apply_part.alloc(need) == cudaSuccess);
+  if (!pass) {
+    cudaGetLastError();   // no room for a pass: vector by vector
+    for (int k = 0; k < n; ++k) bem_gemv(h, x + k * nb, y + k * nb);
+    return;
+  }
+  for (int k = 0, nm; k < n; k += nm) {
+    nm = std::min(kChunk, n - k);
+    if (h->opt.bem_precision == 0 && nm < kChunk) nm = nm >= 4 ? 4 : (nm >= 2 ? 2 : 1);
+    if (nm == 1) bem_gemv(h, x + k * nb, y + k * nb);
+    else bem_pass(h, x + k * nb, y + k * nb, nm, W.apply_part, off);
+  }
+}
+
 // Y = B X for the ensemble (member m at x + m * nb), kChunk members per pass.
 void bem_gemm(nmg_handle *h, const double *x, double *y) {
   Mesh &M = h->mesh;
@@ -2885,10 +2967,6 @@ void bem_gemm(nmg_handle *h, const double *x, double *y) {
     return;
   }
   const int f = (h->opt.bem_precision >= 1 && M.bem32.p) ? 1 : 0;
-  const long long seg = W.gemv_seg[f];
-  const int maxr = W.gemv_maxr[f];
-  const long long Q = M.ld / (f == 0 ? 4 : 8);
-  const long long nwarps = (long long)W.gemv_blocks * (kGemvThreads / 32);
   for (int c0 = 0; c0 < B; c0 += kChunk) {
     const int nm = std::min(kChunk, B - c0);
     const int MB = nm <= 2 ? 2 : (nm <= 4 ? 4 : 8);
@@ -2950,48 +3028,22 @@ void bem_gemm(nmg_handle *h, const double *x, double *y) {
       ++h->launches;
       continue;
     }
-    if (f == 1 && M.bem16lo.p && !h->bem_fp32_only) {   // compensated FP32 pair product on tiles
-      float *xh = reinterpret_cast<float *>(W.bpart.p + W.gemv_x32_off);
-      float *xl = xh + (size_t)nm * M.ld;
-      k_split_x<<<nblk((long long)M.ld * nm, 256), 256, 0, h->stream>>>(nb, M.ld, nm, xc, xh, xl); ++h->launches;
-      const int nslab = (M.ld + kDfCols - 1) / kDfCols;
-      dim3 grid(nslab, (nb + kDfRows - 1) / kDfRows);
-      NMG_PROF_BEGIN(h, 0);
-      if (MB == 2) k_gemm_df<2><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, M.bem16lo, xh, xl, W.bpart);
-      else if (MB == 4) k_gemm_df<4><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, M.bem16lo, xh, xl, W.bpart);
-      else k_gemm_df<8><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, M.bem16lo, xh, xl, W.bpart);
-      NMG_PROF_END(h);
-      ++h->launches;
-      k_slab_sum_m<<<nblk((long long)nb * nm, 256), 256, 0, h->stream>>>(nb, nslab, nm, MB, W.bpart,
-                                                                         y + (size_t)c0 * nb);
-      ++h->launches;
+    if (f == 0 || (M.bem16lo.p && !h->bem_fp32_only)) {   // FP64, or compensated FP32 pairs on tiles
+      bem_pass(h, xc, y + (size_t)c0 * nb, nm, W.bpart, W.gemv_x32_off);
       continue;
     }
-    if (f == 1) {
-      float *x32 = reinterpret_cast<float *>(W.bpart.p + W.gemv_x32_off);
-      k_to_f32_vec<<<nblk((long long)M.ld * nm, 256), 256, 0, h->stream>>>(nb, M.ld, xc, x32, nm); ++h->launches;
-      const int nslab = (M.ld + kRegSlab - 1) / kRegSlab;
-      dim3 grid(nslab, (nb + kRegRows - 1) / kRegRows);
-      NMG_PROF_BEGIN(h, 0);
-      if (MB == 2) k_gemm_f32r<2><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, x32, W.bpart);
-      else if (MB == 4) k_gemm_f32r<4><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, x32, W.bpart);
-      else k_gemm_f32r<8><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, x32, W.bpart);
-      NMG_PROF_END(h);
-      ++h->launches;
-      k_slab_sum_m<<<nblk((long long)nb * nm, 256), 256, 0, h->stream>>>(nb, nslab, nm, MB, W.bpart,
-                                                                         y + (size_t)c0 * nb);
-      ++h->launches;
-      continue;
-    } else {
-      NMG_PROF_BEGIN(h, 0);
-      if (MB == 2) k_gemm_f64<2><<<W.gemv_blocks, kGemvThreads, 0, h->stream>>>(nb, M.ld, seg, maxr, nm, M.bem, xc, W.bpart);
-      else if (MB == 4) k_gemm_f64<4><<<W.gemv_blocks, kGemvThreads, 0, h->stream>>>(nb, M.ld, seg, maxr, nm, M.bem, xc, W.bpart);
-      else k_gemm_f64<8><<<W.gemv_blocks, kGemvThreads, 0, h->stream>>>(nb, M.ld, seg, maxr, nm, M.bem, xc, W.bpart);
-      NMG_PROF_END(h);
-    }
+    float *x32 = reinterpret_cast<float *>(W.bpart.p + W.gemv_x32_off);
+    k_to_f32_vec<<<nblk((long long)M.ld * nm, 256), 256, 0, h->stream>>>(nb, M.ld, xc, x32, nm); ++h->launches;
+    const int nslab = (M.ld + kRegSlab - 1) / kRegSlab;
+    dim3 grid(nslab, (nb + kRegRows - 1) / kRegRows);
+    NMG_PROF_BEGIN(h, 0);
+    if (MB == 2) k_gemm_f32r<2><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, x32, W.bpart);
+    else if (MB == 4) k_gemm_f32r<4><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, x32, W.bpart);
+    else k_gemm_f32r<8><<<grid, 256, 0, h->stream>>>(nb, M.ld, nm, M.bem32, x32, W.bpart);
+    NMG_PROF_END(h);
     ++h->launches;
-    k_row_sum_m<<<nblk((long long)nb * nm, 256), 256, 0, h->stream>>>(nb, Q, seg, maxr, nwarps, nm, MB, W.bpart,
-                                                                      y + (size_t)c0 * nb);
+    k_slab_sum_m<<<nblk((long long)nb * nm, 256), 256, 0, h->stream>>>(nb, nslab, nm, MB, W.bpart,
+                                                                       y + (size_t)c0 * nb);
     ++h->launches;
   }
 }
