@@ -13,19 +13,20 @@
 // swizzle).  The K dimension (the boundary nodes the matrix sums over) is
 // split over CTAs, each accumulating at most kKbPerSplit x 64 terms of every
 // sum in FP32 (the hi.hi term and the five smaller terms in two separate TMEM
-// accumulators); the per-split partial sums are added in FP64, in split
+// accumulators); the per-split partial sums are added in FP32 pairs, in split
 // order, by a second kernel.  So the FP32 accumulation error stays at the
 // level of a thousand terms, not of nb.
 //
 // Tiles: 128 rows of B (one TMEM lane each) x NT right-hand sides (TMEM
-// columns) x 64 entries of K per stage; one thread issues the TMA loads, one
-// the MMAs, four warps read TMEM back.  Every mbarrier wait is bounded; on a
+// columns) x 32 entries of K per stage; one thread issues the TMA loads, one
+// the MMAs, four warps read TMEM back, one tile behind.  Every mbarrier wait is bounded; on a
 // timeout the kernel sets an error flag, stops issuing, waits (bounded) for
 // its own MMAs, frees its TMEM and returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "nmg_internal.h"
@@ -34,8 +35,8 @@ namespace nmg {
 namespace {
 
 // K entries per stage: 32 (rows of 64 bytes, 64-byte swizzle: 4-6 stages
-// fit in shared memory; 0.532 ms per 128-vector film product) or, built with
-// -DNMG_TC_KB=64, 64 (128-byte rows and swizzle, half as many stages; 0.568 ms)
+// fit in shared memory; 0.470 ms per 128-vector film product) or, built with
+// -DNMG_TC_KB=64, 64 (128-byte rows and swizzle, half as many stages; 0.496 ms)
 #ifndef NMG_TC_KB
 #define NMG_TC_KB 32
 #endif
@@ -131,17 +132,28 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // part[(ks * Rstride + n) * Mpad + row]: the FP32 sum over split ks of
 // B[row][k] x_n[k], where plane p of the right-hand sides starts at row
-// p * Rstride of tX.  Grid: (Mpad / 128, ceil(R / NT), splits); 128 threads.
+// p * Rstride of tX.  Persistent: one CTA per SM walks the tiles (row tiles
+// fastest, so that the CTAs at work share a split's right-hand sides in L2),
+// with two tiles' accumulators in TMEM, so that warps 0-3 read one tile back
+// while warp 5 issues the next one's MMAs and warp 4 the loads, whose ring runs
+// on across tiles.  Film, 128 vectors: 470 us (its 2.65 GB of planes take 396) against 540 with a tile per
+// CTA and FP64 adds of the two accumulators (their FP32 sum is the same number:
+// the FP64 one is exact wherever the smaller term counts).
 template <int NT, int ST>
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(192, 1)
     k_bem_tc(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tX, int Mpad, int Rstride,
-             int kb_total, float *__restrict__ part, int *__restrict__ err) {
+             int kb_total, int Mt, int Nt, int tiles, float *__restrict__ part, int *__restrict__ err) {
   constexpr uint32_t kABytes = kTcRows * kTcK * 2, kXBytes = NT * kTcK * 2;
   constexpr uint32_t kStageBytes = 3 * (kABytes + kXBytes);
+  constexpr uint32_t kTmemCols = 4 * NT;   // two tiles' pairs of accumulators: 128, 256 or 512 columns
   extern __shared__ uint8_t dsm_raw[];
-  __shared__ uint64_t full[ST], empty[ST], done;
+  __shared__ uint64_t full[ST], empty[ST], tfull[2], tempty[2], done;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag, n_issued, n_consumed;
   // the six (A plane, X plane) pairs of the split product, largest first
@@ -149,21 +161,20 @@ __global__ void __launch_bounds__(128, 1)
   constexpr int kPairX[6] = {0, 1, 0, 2, 1, 0};
   uint8_t *sm = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(dsm_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kb0 = blockIdx.z * kKbPerSplit;
-  const int nkb = min(kb_total, kb0 + kKbPerSplit) - kb0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int q = 0; q < 2; ++q) { mbar_init(&tfull[q], 1); mbar_init(&tempty[q], 4); }
     mbar_init(&done, 1);
     abort_flag = 0;
     n_issued = n_consumed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // 2 NT TMEM columns (a power of two >= 64): two 128 x NT FP32 accumulators,
-  // columns [0, NT) for the hi.hi term, [NT, 2 NT) for the five smaller ones,
-  // so the small terms' rounding is relative to their own (2^-8 smaller) sums
+  // per tile two 128 x NT FP32 accumulators, columns [0, NT) for the hi.hi
+  // term, [NT, 2 NT) for the five smaller ones, so the small terms' rounding
+  // is relative to their own (2^-8 smaller) sums
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                 "r"((uint32_t)(2 * NT)));
+                 "r"(kTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -173,62 +184,82 @@ __global__ void __launch_bounds__(128, 1)
   volatile int *abort_v = &abort_flag;
   auto tileA = [&](int s, int p) { return sm + (size_t)s * kStageBytes + (size_t)p * kABytes; };
   auto tileX = [&](int s, int p) { return sm + (size_t)s * kStageBytes + 3 * kABytes + (size_t)p * kXBytes; };
+  // K blocks of a tile's split
+  auto blocks = [&](int ks) { return min(kb_total, (ks + 1) * kKbPerSplit) - ks * kKbPerSplit; };
 
-  if (warp == 0 && lane == 0) {   // TMA producer
-    for (int i = 0; i < nkb; ++i) {
-      const int s = i % ST;
-      if (i >= ST && !mbar_wait(&empty[s], ((i / ST) & 1) ^ 1, abort_v)) { *abort_v = 1; break; }
-      mbar_expect_tx(&full[s], kStageBytes);
-      const int kx = (kb0 + i) * kTcK;
-      for (int p = 0; p < 3; ++p) tma_load_2d(tileA(s, p), &tA, kx, p * Mpad + blockIdx.x * kTcRows, &full[s]);
-      for (int p = 0; p < 3; ++p) tma_load_2d(tileX(s, p), &tX, kx, p * Rstride + blockIdx.y * NT, &full[s]);
-      n_issued = i + 1;
+  if (warp == 4 && lane == 0) {   // TMA producer
+    int g = 0;                    // K blocks so far, over all tiles
+    for (int t = blockIdx.x; t < tiles && !*abort_v; t += gridDim.x) {
+      const int mt = t % Mt, q = t / Mt, ntile = q % Nt, ks = q / Nt, nkb = blocks(ks);
+      for (int i = 0; i < nkb; ++i, ++g) {
+        const int s = g % ST;
+        if (g >= ST && !mbar_wait(&empty[s], ((g / ST) & 1) ^ 1, abort_v)) { *abort_v = 1; break; }
+        mbar_expect_tx(&full[s], kStageBytes);
+        const int kx = (ks * kKbPerSplit + i) * kTcK;
+        for (int p = 0; p < 3; ++p) tma_load_2d(tileA(s, p), &tA, kx, p * Mpad + mt * kTcRows, &full[s]);
+        for (int p = 0; p < 3; ++p) tma_load_2d(tileX(s, p), &tX, kx, p * Rstride + ntile * NT, &full[s]);
+        n_issued = g + 1;
+      }
     }
-  } else if (warp == 1 && lane == 0) {   // MMA issuer
+  } else if (warp == 5 && lane == 0) {   // MMA issuer
     constexpr uint32_t idesc = idesc_bf16(kTcRows, NT);
-    for (int i = 0; i < nkb; ++i) {
-      const int s = i % ST;
-      if (!mbar_wait(&full[s], (i / ST) & 1, abort_v)) { *abort_v = 1; break; }
+    int g = 0, it = 0;
+    for (int t = blockIdx.x; t < tiles && !*abort_v; t += gridDim.x, ++it) {
+      const int nkb = blocks(t / Mt / Nt);
+      const uint32_t acc = tmem + (uint32_t)(it & 1) * 2 * NT;
+      if (it >= 2 && !mbar_wait(&tempty[it & 1], ((it >> 1) & 1) ^ 1, abort_v)) { *abort_v = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      uint64_t da[3], dx[3];
-      for (int p = 0; p < 3; ++p) { da[p] = desc_sw(smem_u32(tileA(s, p))); dx[p] = desc_sw(smem_u32(tileX(s, p))); }
+      for (int i = 0; i < nkb; ++i, ++g) {
+        const int s = g % ST;
+        if (!mbar_wait(&full[s], (g / ST) & 1, abort_v)) { *abort_v = 1; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint64_t da[3], dx[3];
+        for (int p = 0; p < 3; ++p) { da[p] = desc_sw(smem_u32(tileA(s, p))); dx[p] = desc_sw(smem_u32(tileX(s, p))); }
 #pragma unroll
-      for (int kk = 0; kk < kTcK / 16; ++kk)   // 16 entries (32 bytes) per MMA: +2 in the encoded address
+        for (int kk = 0; kk < kTcK / 16; ++kk)   // 16 entries (32 bytes) per MMA: +2 in the encoded address
 #pragma unroll
-        for (int t = 0; t < 6; ++t)
-          mma_bf16(t == 0 ? tmem : tmem + NT, da[kPairA[t]] + 2 * kk, dx[kPairX[t]] + 2 * kk, idesc,
-                   (i | kk | (t > 1 ? 1 : 0)) != 0);
-      mma_commit(&empty[s]);   // the stage is free once these MMAs have read it
-      n_consumed = i + 1;
+          for (int q = 0; q < 6; ++q)
+            mma_bf16(q == 0 ? acc : acc + NT, da[kPairA[q]] + 2 * kk, dx[kPairX[q]] + 2 * kk, idesc,
+                     (i | kk | (q > 1 ? 1 : 0)) != 0);
+        mma_commit(&empty[s]);   // the stage is free once these MMAs have read it
+        n_consumed = g + 1;
+      }
+      mma_commit(&tfull[it & 1]);
     }
-    mma_commit(&done);         // tracks every MMA issued above
+    mma_commit(&done);           // tracks every MMA issued above
+  } else if (warp < 4) {         // warp w reads TMEM lanes 32w..32w+31 (rows of the tile)
+    int it = 0;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
+      if (!mbar_wait(&tfull[it & 1], (it >> 1) & 1, abort_v)) { *abort_v = 1; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int mt = t % Mt, q = t / Mt, ntile = q % Nt, ks = q / Nt;
+      const uint32_t acc = tmem + (uint32_t)(it & 1) * 2 * NT + ((uint32_t)(warp * 32) << 16);
+      const int row = mt * kTcRows + warp * 32 + lane;
+      float *out = part + ((size_t)ks * Rstride + (size_t)ntile * NT) * Mpad + row;
+#pragma unroll 1
+      for (int c0 = 0; c0 < NT; c0 += 32) {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(acc + (uint32_t)c0, r0);
+        tmem_ld32(acc + (uint32_t)(NT + c0), r1);
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          out[(size_t)(c0 + j) * Mpad] = __fadd_rn(__uint_as_float(r0[j]), __uint_as_float(r1[j]));
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[it & 1]);
+    }
   }
   __syncwarp();
-  // epilogue: warp w reads TMEM lanes 32w..32w+31 (rows of this tile)
-  const bool ok = mbar_wait(&done, 0, abort_v) && !*abort_v;
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (ok) {
-    const int row = blockIdx.x * kTcRows + warp * 32 + lane;
-    float *out = part + ((size_t)blockIdx.z * Rstride + (size_t)blockIdx.y * NT) * Mpad + row;
-#pragma unroll 1
-    for (int c0 = 0; c0 < NT; c0 += 32) {
-      uint32_t r0[32], r1[32];
-      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r0);
-      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(NT + c0), r1);
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        out[(size_t)(c0 + j) * Mpad] = (float)((double)__uint_as_float(r0[j]) + (double)__uint_as_float(r1[j]));
-    }
-  } else if (threadIdx.x == 0) {
-    atomicOr(err, ERR_BARRIER);
-  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (!ok && threadIdx.x == 32) {   // let the MMAs issued so far finish before the TMEM goes (bounded)
+  const bool ok = !*abort_v;
+  if (!ok && threadIdx.x == 0) atomicOr(err, ERR_BARRIER);
+  if (!ok && threadIdx.x == 160) {   // let the MMAs issued so far finish before the TMEM goes (bounded)
     for (unsigned long long spins = 0; !mbar_try_wait(&done, 0) && spins < kTcSpinLimit; ++spins) {
     }
   }
-  if (!ok && threadIdx.x == 0) {    // and the TMA loads issued but never consumed land before the CTA exits
+  if (!ok && threadIdx.x == 0) {     // and the TMA loads issued but never consumed land before the CTA exits
     for (int i = n_consumed; i < n_issued; ++i)
       for (unsigned long long spins = 0; !mbar_try_wait(&full[i % ST], (i / ST) & 1) && spins < kTcSpinLimit;
            ++spins) {
@@ -236,37 +267,70 @@ __global__ void __launch_bounds__(128, 1)
   }
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * NT)));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-// y[n * nb + row] = sum over the splits, in split order, of the FP32 partials (FP64 adds).
-__global__ void k_tc_reduce(int nb, int R, int Rpad, int Mpad, int splits, const float *__restrict__ part,
-                            double *__restrict__ y) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)R * nb) return;
-  const int n = (int)(idx / nb), row = (int)(idx % nb);
-  double s = 0.0;
-  for (int k = 0; k < splits; ++k) s += (double)__ldcs(part + ((size_t)k * Rpad + n) * Mpad + row);
-  y[idx] = s;
+// y[n * nb + row] = sum over the splits, in split order, of the FP32 partials.
+// The sum is kept as an FP32 pair (TwoSum, the rounding errors in the second
+// part: ~2^-47 of the terms, whose own error is 2^-24) and leaves as FP64: 21
+// conversions and FP64 adds per value made this FP64-pipe-bound (212 us for the
+// film's 128 vectors, 67 now; its 240 MB take 36).
+__global__ void __launch_bounds__(256) k_tc_reduce(int nb, int Rpad, int Mpad, int splits,
+                                                   const float *__restrict__ part, double *__restrict__ y) {
+  const int row = blockIdx.x * blockDim.x + threadIdx.x, n = blockIdx.y;
+  if (row >= nb) return;
+  const float *p = part + (size_t)n * Mpad + row;
+  const size_t stride = (size_t)Rpad * Mpad;
+  float S = 0.f, C = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < splits; ++k) {
+    const float v = __ldcs(p + k * stride);
+    const float s = __fadd_rn(S, v), b = __fsub_rn(s, S);
+    C = __fadd_rn(C, __fadd_rn(__fsub_rn(S, __fsub_rn(s, b)), __fsub_rn(v, b)));
+    S = s;
+  }
+  double sum = (double)S + (double)C;
+  if (!isfinite(sum)) {   // beyond FP32's range, or not finite to begin with
+    sum = 0.0;
+    for (int k = 0; k < splits; ++k) sum += (double)p[k * stride];
+  }
+  y[(size_t)n * nb + row] = sum;
+}
+
+// BF16 rounding of a + e, where |e| is at most half a unit in a's last place:
+// e only decides where a lies halfway between two BF16 numbers.
+__device__ __forceinline__ __nv_bfloat16 bf16_of(float a, float e) {
+  const unsigned u = __float_as_uint(a);
+  if ((u & 0xffffu) == 0x8000u && e != 0.f)
+    return __ushort_as_bfloat16((unsigned short)((u >> 16) + (signbit(a) == signbit(e) ? 1 : 0)));
+  return __float2bfloat16_rn(a);
 }
 
 // Three BF16 planes of a row-major FP64 matrix (rows x cols, row stride lds)
 // into planes of rows padded to rpad and columns to ldk (the pads stay zero).
-__global__ void k_split3_bf16(int rows, int cols, int lds, const double *__restrict__ src, int rpad, int ldk,
-                              __nv_bfloat16 *__restrict__ dst) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)rows * cols) return;
-  const int r = (int)(idx / cols), c = (int)(idx % cols);
-  const double v = src[(size_t)r * lds + c];
-  const __nv_bfloat16 hi = __double2bfloat16(v);
-  const double r1 = v - (double)__bfloat162float(hi);
-  const __nv_bfloat16 mid = __double2bfloat16(r1);
-  const double r2 = r1 - (double)__bfloat162float(mid);
-  const __nv_bfloat16 lo = __double2bfloat16(r2);
-  const size_t plane = (size_t)rpad * ldk, at = (size_t)r * ldk + c;
-  dst[at] = hi;
-  dst[plane + at] = mid;
-  dst[2 * plane + at] = lo;
+// Each plane is the BF16 rounding of what the ones before leave; the value is
+// first taken apart into two FP32 numbers, so that three FP64 instructions
+// remain of the seven that held this up (film, 128 vectors: 36 -> 22 us).
+__global__ void __launch_bounds__(256) k_split3_bf16(int rows, int cols, int lds, const double *__restrict__ src,
+                                                     int rpad, int ldk, __nv_bfloat16 *__restrict__ dst) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  const size_t plane = (size_t)rpad * ldk;
+  for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+    const double v = src[(size_t)r * lds + c];
+    const float f = (float)v, e = (float)(v - (double)f);
+    const __nv_bfloat16 hi = bf16_of(f, e);
+    const float r1 = f - __bfloat162float(hi);            // exact, like the next differences
+    const float s1 = r1 + e, e1 = e - (s1 - r1);
+    const __nv_bfloat16 mid = bf16_of(s1, e1);
+    const float r2 = s1 - __bfloat162float(mid);
+    const float s2 = r2 + e1, e2 = e1 - (s2 - r2);
+    const __nv_bfloat16 lo = bf16_of(s2, e2);
+    const size_t at = (size_t)r * ldk + c;
+    dst[at] = hi;
+    dst[plane + at] = mid;
+    dst[2 * plane + at] = lo;
+  }
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -313,8 +377,7 @@ int bem_tc_setup(nmg_handle *h, std::string &err) {
   const size_t plane = (size_t)T.Mpad * T.ldk;
   NMG_CUDA_TRY(T.bplanes.alloc(3 * plane), "alloc BF16 BEM planes");
   NMG_CUDA_TRY(cudaMemsetAsync(T.bplanes.p, 0, sizeof(uint16_t) * 3 * plane, h->stream), "zero BF16 planes");
-  const long long n = (long long)nb * nb;
-  k_split3_bf16<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(
+  k_split3_bf16<<<dim3((nb + 255) / 256, std::min(nb, 32768)), 256, 0, h->stream>>>(
       nb, nb, M.ld, M.bem, T.Mpad, T.ldk, reinterpret_cast<__nv_bfloat16 *>(T.bplanes.p));
   ++h->launches;
   NMG_CUDA_TRY(cudaGetLastError(), "split BEM planes");
@@ -366,35 +429,33 @@ int bem_tc(nmg_handle *h, const double *x, double *y, int R) {
     return 100;
   }
   const int NT = T.nt, Rpad = T.Rcap;   // Rpad: the planes' row stride (rows >= R are never read back)
-  const long long n = (long long)R * nb;
-  k_split3_bf16<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(
+  k_split3_bf16<<<dim3((nb + 255) / 256, std::min(R, 32768)), 256, 0, h->stream>>>(
       R, nb, nb, x, Rpad, T.ldk, reinterpret_cast<__nv_bfloat16 *>(T.xplanes.p));
   ++h->launches;
   const int kb_total = T.ldk / kTcK;
   const int splits = (kb_total + kKbPerSplit - 1) / kKbPerSplit;
-  const dim3 grid(T.Mpad / kTcRows, (R + NT - 1) / NT, splits);
+  const int Mt = T.Mpad / kTcRows, Nt = (R + NT - 1) / NT, tiles = Mt * Nt * splits;
+  const dim3 grid(std::min(tiles, h->sm_count));
   const CUtensorMap &mA = *reinterpret_cast<const CUtensorMap *>(T.mapA);
   const CUtensorMap &mX = *reinterpret_cast<const CUtensorMap *>(T.mapX);
+  auto launch = [&](auto kernel, size_t sm) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    kernel<<<grid, 192, sm, h->stream>>>(mA, mX, T.Mpad, Rpad, kb_total, Mt, Nt, tiles, T.part, h->ws.err);
+  };
   {
     NMG_PROF_BEGIN(h, 0);
-    if (NT == 32) {
-      const size_t sm = tc_smem<32, 3 * kStMul>();
-      cudaFuncSetAttribute(k_bem_tc<32, 3 * kStMul>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_bem_tc<32, 3 * kStMul><<<grid, 128, sm, h->stream>>>(mA, mX, T.Mpad, Rpad, kb_total, T.part, h->ws.err);
-    } else if (NT == 64) {
-      const size_t sm = tc_smem<64, 3 * kStMul>();
-      cudaFuncSetAttribute(k_bem_tc<64, 3 * kStMul>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_bem_tc<64, 3 * kStMul><<<grid, 128, sm, h->stream>>>(mA, mX, T.Mpad, Rpad, kb_total, T.part, h->ws.err);
-    } else {
-      const size_t sm = tc_smem<128, 2 * kStMul>();
-      cudaFuncSetAttribute(k_bem_tc<128, 2 * kStMul>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_bem_tc<128, 2 * kStMul><<<grid, 128, sm, h->stream>>>(mA, mX, T.Mpad, Rpad, kb_total, T.part, h->ws.err);
-    }
+    if (NT == 32) launch(k_bem_tc<32, 3 * kStMul>, tc_smem<32, 3 * kStMul>());
+    else if (NT == 64) launch(k_bem_tc<64, 3 * kStMul>, tc_smem<64, 3 * kStMul>());
+    else launch(k_bem_tc<128, 2 * kStMul>, tc_smem<128, 2 * kStMul>());
     ++h->launches;
     NMG_PROF_END(h);
   }
-  k_tc_reduce<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(nb, R, Rpad, T.Mpad, splits, T.part, y);
-  ++h->launches;
+  for (int n0 = 0; n0 < R; n0 += 32768) {   // grid.y ends at 65,535
+    const int nr = std::min(32768, R - n0);
+    k_tc_reduce<<<dim3((nb + 255) / 256, nr), 256, 0, h->stream>>>(nb, Rpad, T.Mpad, splits,
+                                                                  T.part + (size_t)n0 * T.Mpad, y + (size_t)n0 * nb);
+    ++h->launches;
+  }
   if (cudaGetLastError() != cudaSuccess) {
     h->last_error = "bem_tc: launch failed";
     return 100;
