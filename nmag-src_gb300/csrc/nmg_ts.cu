@@ -18,8 +18,10 @@
 //   Hv = -c_exch K v / V_i,  with (m, H_total) frozen at the last re-Jacobi.
 // Preconditioner: exact inverse of each node's 3x3 block of I - gamma J
 // (gamma of the last setup, as the reference's cached KSP).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "nmg_internal.h"
@@ -40,10 +42,6 @@ constexpr int kRedBlocks = 304;   // two blocks per SM: enough loads in flight f
 
 inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
-__device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
 // ---- elementwise kernels ----
 __global__ void k_lin(int n, double a, const double *__restrict__ x, double b, const double *__restrict__ y,
@@ -66,16 +64,30 @@ __global__ void k_ewt(int n, double rtol, double atol, const double *__restrict_
   ws[i] = sc;
 }
 struct ZnPtrs { double *z[QMAXB + 2]; };
-// Nordsieck prediction z <- z * Pascal (sign = +1) or its inverse (sign = -1).
+// Nordsieck prediction z <- z * Pascal (sign = +1) or its inverse (sign = -1);
+// before it, where asked for, the error weights from zn0 (w != null: k_ewt) and
+// the rescaling z_j *= eta^j of a changed step (eta != 1), in one pass.
 // (The order q is a template parameter: with compile-time indices the
 // history pointers and values stay in registers.)
 template <int Q>
-__global__ void k_predict(int n, ZnPtrs zn, int sign) {
+__global__ void k_predict(int n, ZnPtrs zn, int sign, double eta, double rtol, double atol, double *__restrict__ w,
+                          double *__restrict__ ws) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double v[Q + 1];
 #pragma unroll
   for (int j = 0; j <= Q; ++j) v[j] = zn.z[j][i];
+  if (w) {
+    const double sc = rtol * fabs(v[0]) + atol;
+    w[i] = 1.0 / sc;
+    ws[i] = sc;
+  }
+  if (eta != 1.0) {
+    double f = eta;
+#pragma unroll
+    for (int j = 1; j <= Q; ++j) { v[j] = __dmul_rn(v[j], f); f *= eta; }
+    zn.z[Q][i] = v[Q];
+  }
 #pragma unroll
   for (int k = 1; k <= Q; ++k)
 #pragma unroll
@@ -83,22 +95,16 @@ __global__ void k_predict(int n, ZnPtrs zn, int sign) {
 #pragma unroll
   for (int j = 0; j < Q; ++j) zn.z[j][i] = v[j];
 }
-template <int Q>
-__global__ void k_rescale(int n, ZnPtrs zn, double eta) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double f = eta;
-#pragma unroll
-  for (int j = 1; j <= Q; ++j) { zn.z[j][i] *= f; f *= eta; }
-}
 struct Coef { double c[QMAXB + 2]; };
+// zn_j += l_j acor; save: where the correction is kept (zn[qmax] of a coming order raise) or null
 template <int Q>
-__global__ void k_complete(int n, ZnPtrs zn, Coef l, const double *__restrict__ acor) {
+__global__ void k_complete(int n, ZnPtrs zn, Coef l, const double *__restrict__ acor, double *save) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double a = acor[i];
 #pragma unroll
   for (int j = 0; j <= Q; ++j) zn.z[j][i] += l.c[j] * a;
+  if (save) save[i] = a;
 }
 // launch K<q>(args...) for the runtime order q in [1, QMAXB]
 #define NMG_LAUNCH_Q(K, q, grid, blk, st, ...)                            \
@@ -119,25 +125,17 @@ __global__ void k_interp(int n, int q, ZnPtrs zn, double s, double *__restrict__
   for (int j = q - 1; j >= 0; --j) v = zn.z[j][i] + s * v;
   out[i] = v;
 }
-// Newton residual: tempv = gamma f - (rl1 zn1 + acor)
-__global__ void k_newton_res(int n, double gamma, const double *__restrict__ f, double rl1,
-                             const double *__restrict__ zn1, const double *__restrict__ acor, double *__restrict__ t) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) t[i] = gamma * f[i] - (rl1 * zn1[i] + acor[i]);
-}
-// acor += b ; y = zn0 + acor
-__global__ void k_newton_upd(int n, const double *__restrict__ b, double *__restrict__ acor,
-                             const double *__restrict__ zn0, double *__restrict__ y) {
+// A Krylov vector scaled by a, and the direction t = v / w it is applied to
+// (ws = 1 / w; t32: the FP32 form's direction): the division in its own pass,
+// inside the FP64-bound Jv kernel it would be repeated for every neighbour.
+__global__ void k_scale_dir(int n, double a, double *__restrict__ v, const double *__restrict__ ws,
+                            double *__restrict__ t, float *__restrict__ t32) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double a = acor[i] + b[i];
-  acor[i] = a;
-  y[i] = zn0[i] + a;
-}
-// o = v / w, given ws = 1 / w
-__global__ void k_div_ewt(int n, const double *__restrict__ v, const double *__restrict__ ws, double *__restrict__ o) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) o[i] = v[i] * ws[i];
+  const double x = v[i] * a;
+  v[i] = x;
+  if (t32) t32[i] = (float)(x * ws[i]);
+  else t[i] = x * ws[i];
 }
 __global__ void k_hub(int n, const double *__restrict__ y, const double *__restrict__ yp, const double *__restrict__ w,
                       double *__restrict__ out) {
@@ -145,19 +143,89 @@ __global__ void k_hub(int n, const double *__restrict__ y, const double *__restr
   if (i < n) out[i] = fabs(yp[i]) / (0.1 * fabs(y[i]) + 1.0 / w[i]);
 }
 
-// ---- reductions: block partials then one ordered final sum on the host ----
-// mode 0: sum (x w)^2 ; mode 1: sum x y ; mode 2: max x
-__global__ void k_red(int n, int mode, const double *__restrict__ x, const double *__restrict__ y,
-                      double *__restrict__ part) {
-  __shared__ double sm[32];
-  double acc = 0.0;
+// ---- reductions ----
+// Sums over the grid in one launch: the blocks' partials (in a fixed order, so
+// a sum does not depend on timing) are added by the block that finishes last.
+// Its results go to the device (out) and, where the host decides on them, to
+// pinned memory followed by a sequence number that the host waits for: a
+// separate final kernel took 9.5 us, and the copy and stream synchronisation
+// of a readback ~15 us each, in a step whose field evaluation takes 130
+// (cube, 1,331 nodes).
+struct Red {
+  double *part;               // kRedMax x gridDim.x partials
+  unsigned *count;            // blocks done; 0 between launches
+  double *host;               // pinned results, or null
+  unsigned long long *flag;   // pinned sequence number
+  unsigned long long seq;
+};
+constexpr int kRedMax = 32;
+
+// v[0..nv) summed (or, kMax, their largest against 0) over the grid; true in the
+// last block, where tot(k, value) has been called by one thread for each k.
+template <int K, bool kMax = false, class F>
+__device__ __forceinline__ bool red_grid(const double (&v)[K], int nv, const Red &r, F tot) {
+  __shared__ double sm[8][K];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto tree = [](double x) {
+    for (int o = 16; o; o >>= 1) {
+      const double z = __shfl_xor_sync(0xffffffffu, x, o);
+      x = kMax ? fmax(x, z) : x + z;
+    }
+    return x;
+  };
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (k >= nv) break;
+    const double s = tree(v[k]);
+    if (lane == 0) sm[wid][k] = s;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < nv) {
+    double s = 0.0;
+    for (int w = 0; w < 8; ++w) s = kMax ? fmax(s, sm[w][threadIdx.x]) : s + sm[w][threadIdx.x];
+    __stcg(r.part + (size_t)threadIdx.x * gridDim.x + blockIdx.x, s);
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(r.count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  for (int k = wid; k < nv; k += 8) {
+    double s = 0.0;
+#pragma unroll 4
+    for (int b = lane; b < (int)gridDim.x; b += 32) {
+      const double x = __ldcg(r.part + (size_t)k * gridDim.x + b);
+      s = kMax ? fmax(s, x) : s + x;
+    }
+    s = tree(s);
+    if (lane == 0) tot(k, s);
+  }
+  if (threadIdx.x == 0) *r.count = 0;
+  return true;
+}
+// After the writes to r.host by any threads of the block: the host may read them.
+__device__ __forceinline__ void red_post(const Red &r) {
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    *(volatile unsigned long long *)r.flag = r.seq;
+  }
+}
+
+// mode 0: sum (x w)^2 ; mode 1: sum x y ; mode 2: max x -> r.host[0]
+template <int kMode>
+__global__ void __launch_bounds__(256) k_red(int n, const double *__restrict__ x, const double *__restrict__ y, Red r) {
+  double acc[1] = {0.0};
   const int stride = gridDim.x * blockDim.x;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   auto step = [&](double xv, double yv) {
     const double v = xv * yv;
-    if (mode == 0) acc += v * v;
-    else if (mode == 1) acc += v;
-    else acc = fmax(acc, xv);
+    if (kMode == 0) acc[0] += v * v;
+    else if (kMode == 1) acc[0] += v;
+    else acc[0] = fmax(acc[0], xv);
   };
   for (; i + 3 * stride < n; i += 4 * stride) {   // four loads of each vector in flight, same order
     const double x0 = x[i], x1 = x[i + stride], x2 = x[i + 2 * stride], x3 = x[i + 3 * stride];
@@ -165,73 +233,49 @@ __global__ void k_red(int n, int mode, const double *__restrict__ x, const doubl
     step(x0, y0); step(x1, y1); step(x2, y2); step(x3, y3);
   }
   for (; i < n; i += stride) step(x[i], y[i]);
-  if (mode == 2) { for (int o = 16; o; o >>= 1) acc = fmax(acc, __shfl_xor_sync(0xffffffffu, acc, o)); }
-  else acc = warp_sum(acc);
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s = (mode == 2) ? fmax(s, sm[w]) : s + sm[w];
-    part[blockIdx.x] = s;
-  }
+  if (red_grid<1, kMode == 2>(acc, 1, r, [&](int, double s) { r.host[0] = s; })) red_post(r);
 }
-// Multi-dot h[k] = V[k] . w for k < nv (Gram-Schmidt), partials per block.
-struct VecPtrs { const double *v[32]; };
+
+struct VecPtrs { const double *v[kRedMax]; };
+// Multi-dot h[k] = V[k] . w for k < nv (Gram-Schmidt), and hcol, the Hessenberg
+// column summed over the passes.  With kOrth, w has first the components given
+// by h taken out (the pass before), V's values being read once for both.
 // NVM: compile-time bound on nv (the accumulators and vector pointers stay
 // in registers).
-template <int NVM>
-__global__ void k_mdot(int n, int nv, VecPtrs V, const double *__restrict__ w, double *__restrict__ part) {
-  __shared__ double sm[32][33];
+template <int NVM, bool kOrth>
+__global__ void __launch_bounds__(256) k_mdot(int n, int nv, VecPtrs V, double *__restrict__ w, double *h,
+                                              double *__restrict__ hcol, int first, Red r) {
+  __shared__ double hs[NVM];
+  if (kOrth) {
+    if ((int)threadIdx.x < nv) hs[threadIdx.x] = h[threadIdx.x];
+    __syncthreads();
+  }
   double acc[NVM];
 #pragma unroll
   for (int k = 0; k < NVM; ++k) acc[k] = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double wi = w[i];
+    double wi = w[i], vk[NVM];
 #pragma unroll
-    for (int k = 0; k < NVM; ++k) if (k < nv) acc[k] += V.v[k][i] * wi;
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int k = 0; k < NVM; ++k) vk[k] = k < nv ? V.v[k][i] : 0.0;
+    if (kOrth) {
 #pragma unroll
-  for (int k = 0; k < NVM; ++k) {
-    if (k >= nv) break;
-    double s = warp_sum(acc[k]);
-    if (lane == 0) sm[wid][k] = s;
+      for (int k = 0; k < NVM; ++k) if (k < nv) wi -= hs[k] * vk[k];
+      w[i] = wi;
+    }
+#pragma unroll
+    for (int k = 0; k < NVM; ++k) if (k < nv) acc[k] += vk[k] * wi;
   }
-  __syncthreads();
-  if (threadIdx.x < nv) {
-    double s = 0.0;
-    for (int wv = 0; wv < (int)(blockDim.x >> 5); ++wv) s += sm[wv][threadIdx.x];
-    part[(size_t)blockIdx.x * 32 + threadIdx.x] = s;
-  }
+  // every block has read h before the last one writes it
+  red_grid<NVM>(acc, nv, r, [&](int k, double s) {
+    h[k] = s;
+    hcol[k] = first ? s : hcol[k] + s;
+  });
 }
-// Ordered sum of the multi-dot partials into h (device), one block of 256
-// threads: thread (chunk c = tid / 32, value k = tid % 32) adds the partials
-// of blocks [c * nblocks / 8, (c + 1) * nblocks / 8) in order, then thread k
-// adds the 8 chunk sums in order.
-__global__ void __launch_bounds__(256) k_mdot_final(int nblocks, int nv, const double *__restrict__ part,
-                                                    double *__restrict__ h, double *__restrict__ hcol, int first) {
-  __shared__ double sc[8][32];
-  const int k = threadIdx.x & 31, c = threadIdx.x >> 5;
-  const int b0 = (int)((long long)c * nblocks / 8), b1 = (int)((long long)(c + 1) * nblocks / 8);
-  double s = 0.0;
-  if (k < nv) {
-#pragma unroll 8
-    for (int b = b0; b < b1; ++b) s += part[(size_t)b * 32 + k];
-  }
-  sc[c][k] = s;
-  __syncthreads();
-  if (threadIdx.x < nv) {
-    double t = 0.0;
-#pragma unroll
-    for (int cc = 0; cc < 8; ++cc) t += sc[cc][threadIdx.x];
-    h[threadIdx.x] = t;
-    hcol[threadIdx.x] = first ? t : hcol[threadIdx.x] + t;   // the Hessenberg column, summed over the passes
-  }
-}
+// w -= sum_k h_k V_k
 template <int NVM>
 __global__ void k_orth(int n, int nv, VecPtrs V, const double *__restrict__ h, double *__restrict__ w) {
-  __shared__ double hs[32];
-  if (threadIdx.x < nv) hs[threadIdx.x] = h[threadIdx.x];
+  __shared__ double hs[NVM];
+  if ((int)threadIdx.x < nv) hs[threadIdx.x] = h[threadIdx.x];
   __syncthreads();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -240,9 +284,31 @@ __global__ void k_orth(int n, int nv, VecPtrs V, const double *__restrict__ h, d
   for (int k = 0; k < NVM; ++k) if (k < nv) s -= hs[k] * V.v[k][i];
   w[i] = s;
 }
+// k_orth, then |w|^2 and the nh entries of the Hessenberg column for the host:
+// r.host[0..nh) and r.host[nh].  nv = 0 leaves w as it is.
+template <int NVM>
+__global__ void __launch_bounds__(256) k_orth_norm(int n, int nv, VecPtrs V, const double *__restrict__ h,
+                                                   double *__restrict__ w, int nh, const double *__restrict__ hcol,
+                                                   Red r) {
+  __shared__ double hs[NVM];
+  if ((int)threadIdx.x < nv) hs[threadIdx.x] = h[threadIdx.x];
+  __syncthreads();
+  double acc[1] = {0.0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double s = w[i];
+#pragma unroll
+    for (int k = 0; k < NVM; ++k) if (k < nv) s -= hs[k] * V.v[k][i];
+    if (nv) w[i] = s;
+    acc[0] += s * s;
+  }
+  if (red_grid<1>(acc, 1, r, [&](int, double s) { r.host[nh] = s; })) {
+    for (int k = threadIdx.x; k < nh; k += blockDim.x) r.host[k] = hcol[k];
+    red_post(r);
+  }
+}
 // x += sum_k c_k V_k with the coefficients passed by value (no host-to-device
 // copy, so the host need not wait before reusing its buffer)
-struct Coef32 { double c[32]; };
+struct Coef32 { double c[kRedMax]; };
 template <int NVM>
 __global__ void k_axpy_multi(int n, int nv, VecPtrs V, Coef32 c, double *__restrict__ x) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -252,58 +318,80 @@ __global__ void k_axpy_multi(int n, int nv, VecPtrs V, Coef32 c, double *__restr
   for (int k = 0; k < NVM; ++k) if (k < nv) s -= (-c.c[k]) * V.v[k][i];
   x[i] = s;
 }
-void launch_axpy_multi(int n, int nv, const VecPtrs &vp, const Coef32 &c, double *x, cudaStream_t st) {
-  const int g = nblk(n, 256);
-  if (nv <= 1) k_axpy_multi<1><<<g, 256, 0, st>>>(n, nv, vp, c, x);
-  else if (nv <= 2) k_axpy_multi<2><<<g, 256, 0, st>>>(n, nv, vp, c, x);
-  else if (nv <= 4) k_axpy_multi<4><<<g, 256, 0, st>>>(n, nv, vp, c, x);
-  else if (nv <= 8) k_axpy_multi<8><<<g, 256, 0, st>>>(n, nv, vp, c, x);
-  else if (nv <= 16) k_axpy_multi<16><<<g, 256, 0, st>>>(n, nv, vp, c, x);
-  else k_axpy_multi<32><<<g, 256, 0, st>>>(n, nv, vp, c, x);
-}
-// k_orth followed by the block partials of |w|^2, in k_red's grid, order and
-// tree (mode 1), so the norm is the same number k_red would give.
-template <int NVM>
-__global__ void k_orth_norm(int n, int nv, VecPtrs V, const double *__restrict__ h, double *__restrict__ w,
-                            double *__restrict__ part) {
-  __shared__ double hs[32], sm[32];
-  if (threadIdx.x < nv) hs[threadIdx.x] = h[threadIdx.x];
-  __syncthreads();
-  double acc = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double s = w[i];
+// Start of a Newton iteration, a node per thread: the residual
+// t = gamma f - (rl1 zn1 + acor), its preconditioned form
+// v0 = ewt P^{-1} t, and the sums (t ewt)^2 and v0^2 for the host.  The first
+// iteration's acor = 0 and y = zn0 are written here.
+__global__ void __launch_bounds__(256)
+    k_newton_start(int nodes, int first, double gamma, const double *__restrict__ f, double rl1,
+                   const double *__restrict__ zn0, const double *__restrict__ zn1, double *__restrict__ acor,
+                   double *__restrict__ y, const double *__restrict__ Pinv, const double *__restrict__ ewt,
+                   double *__restrict__ t, double *__restrict__ v0, Red r) {
+  double acc[2] = {0.0, 0.0};
+  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < nodes; g += gridDim.x * blockDim.x) {
+    const size_t o = 3 * (size_t)g;
+    const double *Pi = Pinv + 9 * (size_t)g;
+    double ri[3], e[3];
 #pragma unroll
-    for (int k = 0; k < NVM; ++k) if (k < nv) s -= hs[k] * V.v[k][i];
-    w[i] = s;
-    const double v = s * s;
-    acc += v;
+    for (int d = 0; d < 3; ++d) {
+      double a = 0.0;
+      if (first) {
+        acor[o + d] = 0.0;
+        y[o + d] = zn0[o + d];
+      } else a = acor[o + d];
+      ri[d] = gamma * f[o + d] - (rl1 * zn1[o + d] + a);
+      t[o + d] = ri[d];
+      e[d] = ewt[o + d];
+      const double q = ri[d] * e[d];
+      acc[0] += q * q;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double q = e[d] * ((Pi[3 * d] * ri[0] + Pi[3 * d + 1] * ri[1]) + Pi[3 * d + 2] * ri[2]);
+      v0[o + d] = q;
+      acc[1] += q * q;
+    }
   }
-  acc = warp_sum(acc);
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int wv = 0; wv < (int)(blockDim.x >> 5); ++wv) t = t + sm[wv];
-    part[blockIdx.x] = t;
+  if (red_grid<2>(acc, 2, r, [&](int k, double s) { r.host[k] = s; })) red_post(r);
+}
+// End of one: the correction b = (x0 + sum_k c_k V_k) / ewt (x0 null: 0) or, kRes,
+// b = x0 as it is; acor += b, y = zn0 + acor, and the sum (b ewt)^2 for the host.
+template <int NVM>
+__global__ void __launch_bounds__(256)
+    k_newton_end(int n, int nv, VecPtrs V, Coef32 c, const double *__restrict__ x0, int res,
+                 const double *__restrict__ ewt, const double *__restrict__ ews, const double *__restrict__ zn0,
+                 double *__restrict__ acor, double *__restrict__ y, Red r) {
+  double acc[1] = {0.0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double s = x0 ? x0[i] : 0.0;
+#pragma unroll
+    for (int k = 0; k < NVM; ++k) if (k < nv) s -= (-c.c[k]) * V.v[k][i];
+    if (!res) s *= ews[i];
+    const double q = s * ewt[i], a = acor[i] + s;
+    acc[0] += q * q;
+    acor[i] = a;
+    y[i] = zn0[i] + a;
   }
+  if (red_grid<1>(acc, 1, r, [&](int, double t) { r.host[0] = t; })) red_post(r);
 }
-void launch_orth_norm(int n, int nv, const VecPtrs &vp, const double *h, double *w, double *part, cudaStream_t st) {
-  if (nv <= 1) k_orth_norm<1><<<kRedBlocks, 256, 0, st>>>(n, nv, vp, h, w, part);
-  else if (nv <= 2) k_orth_norm<2><<<kRedBlocks, 256, 0, st>>>(n, nv, vp, h, w, part);
-  else if (nv <= 4) k_orth_norm<4><<<kRedBlocks, 256, 0, st>>>(n, nv, vp, h, w, part);
-  else if (nv <= 8) k_orth_norm<8><<<kRedBlocks, 256, 0, st>>>(n, nv, vp, h, w, part);
-  else if (nv <= 16) k_orth_norm<16><<<kRedBlocks, 256, 0, st>>>(n, nv, vp, h, w, part);
-  else k_orth_norm<32><<<kRedBlocks, 256, 0, st>>>(n, nv, vp, h, w, part);
+// F.template operator()<NVM>() for the smallest NVM >= nv
+template <class F>
+void with_nvm(int nv, F f) {
+  if (nv <= 1) f(std::integral_constant<int, 1>());
+  else if (nv <= 2) f(std::integral_constant<int, 2>());
+  else if (nv <= 4) f(std::integral_constant<int, 4>());
+  else if (nv <= 8) f(std::integral_constant<int, 8>());
+  else if (nv <= 16) f(std::integral_constant<int, 16>());
+  else f(std::integral_constant<int, 32>());
 }
-// k_orth<NVM> for the smallest NVM >= nv
-void launch_orth(int n, int nv, const VecPtrs &vp, const double *h, double *w, cudaStream_t st) {
-  const int g = nblk(n, 256);
-  if (nv <= 1) k_orth<1><<<g, 256, 0, st>>>(n, nv, vp, h, w);
-  else if (nv <= 2) k_orth<2><<<g, 256, 0, st>>>(n, nv, vp, h, w);
-  else if (nv <= 4) k_orth<4><<<g, 256, 0, st>>>(n, nv, vp, h, w);
-  else if (nv <= 8) k_orth<8><<<g, 256, 0, st>>>(n, nv, vp, h, w);
-  else if (nv <= 16) k_orth<16><<<g, 256, 0, st>>>(n, nv, vp, h, w);
-  else k_orth<32><<<g, 256, 0, st>>>(n, nv, vp, h, w);
+// Blocks of a reduction over n values, a thread each, up to kRedBlocks
+inline int red_blocks(int n) { return std::min(kRedBlocks, nblk(n, 256)); }
+// classical RK4's update m += dt/6 (k1 + 2 k2 + 2 k3 + k4)
+__global__ void k_rk4(int n, double c, const double *__restrict__ k1, const double *__restrict__ k2,
+                      const double *__restrict__ k3, const double *__restrict__ k4, double *__restrict__ m) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  m[i] += c * (((k1[i] + 2.0 * k2[i]) + 2.0 * k3[i]) + k4[i]);
 }
 
 // The local terms of dF/dm . w beyond the exchange (Jacobian level >= 1):
@@ -526,11 +614,6 @@ __global__ void k_jv32(Jv32Args a) {
   }
 }
 
-// t32 = (float)(v / ewt): the FP32 direction of k_jv32
-__global__ void k_div_ewt32(int n, const double *__restrict__ v, const double *__restrict__ ws, float *__restrict__ o) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) o[i] = (float)(v[i] * ws[i]);
-}
 
 __global__ void k_to_f32(long long n, const double *__restrict__ x, float *__restrict__ y) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -584,18 +667,6 @@ __global__ void k_pprep(int N, const int32_t *__restrict__ diag_pos, const doubl
   }
 }
 
-// Block-Jacobi preconditioner alone: out = ewt * P^{-1} r (r unscaled).
-__global__ void k_psolve(long long n3, const double *__restrict__ Pinv, const double *__restrict__ r,
-                         const double *__restrict__ ewt, double *__restrict__ out) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (3 * g >= n3) return;
-  const double *Pi = Pinv + 9 * (size_t)g, *ri = r + 3 * (size_t)g;
-  for (int d = 0; d < 3; ++d) {
-    size_t o = 3 * (size_t)g + d;
-    out[o] = ewt[o] * ((Pi[3 * d] * ri[0] + Pi[3 * d + 1] * ri[1]) + Pi[3 * d + 2] * ri[2]);
-  }
-}
-
 }  // namespace
 
 struct Integrator {
@@ -610,7 +681,11 @@ struct Integrator {
   DevBuf<double> ewts;   // 1 / ewt
   double *zn[QMAXB + 2];
   std::vector<double *> V;
-  double *hpin = nullptr;  // pinned readback
+  DevBuf<unsigned> redcnt;
+  double *hpin = nullptr;  // pinned results of the reductions, after the sequence number's line
+  unsigned long long seq = 0;
+  double eta_due = 1.0;    // the next prediction rescales the history by this
+  bool ewt_due = false;    // and forms the error weights first
   // CVODE state
   double tn = 0, h = 0, hprime = 0, eta = 1, hscale = 0, etamax = ETAMX1, rl1 = 1, gamma = 0, gammap = 0,
          gamrat = 1, crate = 1, acnrm = 0, nlscoef = CORTES, saved_tq5 = 0, beta0 = 0;
@@ -625,21 +700,31 @@ struct Integrator {
   cudaStream_t s() const { return hd->stream; }
   ZnPtrs znp() const { ZnPtrs z; for (int j = 0; j < QMAXB + 2; ++j) z.z[j] = zn[j]; return z; }
 
+  double *res() const { return hpin + 8; }
+  Red red(bool host = true) {
+    if (host) ++seq;
+    return Red{part.p, redcnt.p, res(), reinterpret_cast<unsigned long long *>(hpin), seq};
+  }
+  // Waits for the last reduction's results; false if its kernel did not run.
+  bool wait() {
+    for (unsigned spins = 1;; ++spins) {
+      if (__atomic_load_n(reinterpret_cast<unsigned long long *>(hpin), __ATOMIC_ACQUIRE) == seq) return true;
+      if (spins & 0xfff) continue;
+      const cudaError_t e = cudaStreamQuery(s());   // a launch that failed never posts
+      if (e != cudaErrorNotReady)
+        return e == cudaSuccess &&
+               __atomic_load_n(reinterpret_cast<unsigned long long *>(hpin), __ATOMIC_ACQUIRE) == seq;
+    }
+  }
   double wrms(const double *x, const double *w) {
-    k_red<<<kRedBlocks, 256, 0, s()>>>(n, 0, x, w, part); ++hd->launches;
-    cudaMemcpyAsync(hpin, part.p, sizeof(double) * kRedBlocks, cudaMemcpyDeviceToHost, s());
-    if (cudaStreamSynchronize(s()) != cudaSuccess) { status = 100; return 0.0; }
-    double acc = 0.0;
-    for (int b = 0; b < kRedBlocks; ++b) acc += hpin[b];
-    return std::sqrt(acc / n);
+    k_red<0><<<red_blocks(n), 256, 0, s()>>>(n, x, w, red()); ++hd->launches;
+    if (!wait()) { status = 100; return 0.0; }
+    return std::sqrt(res()[0] / n);
   }
   double maxval(const double *x) {
-    k_red<<<kRedBlocks, 256, 0, s()>>>(n, 2, x, x, part); ++hd->launches;
-    cudaMemcpyAsync(hpin, part.p, sizeof(double) * kRedBlocks, cudaMemcpyDeviceToHost, s());
-    if (cudaStreamSynchronize(s()) != cudaSuccess) { status = 100; return 0.0; }
-    double mx = 0.0;
-    for (int b = 0; b < kRedBlocks; ++b) mx = hpin[b] > mx ? hpin[b] : mx;
-    return mx;
+    k_red<2><<<red_blocks(n), 256, 0, s()>>>(n, x, x, red()); ++hd->launches;
+    if (!wait()) { status = 100; return 0.0; }
+    return res()[0];
   }
   void lin(double a, const double *x, double b, const double *yv, double *z) {
     k_lin<<<nblk(n, 256), 256, 0, s()>>>(n, a, x, b, yv, z); ++hd->launches;
@@ -766,76 +851,64 @@ JvArgs jv_args(Integrator &I, const double *t, double *out, int psolve) {
   return a;
 }
 
-// Gram-Schmidt of w against V[0..nv): two classical passes (CGS2); the
-// coefficients stay on the device in hcol.
-// Returns true when the second pass also left the block partials of |w|^2
-// in I.part (nv <= 32: one chunk).
-bool orthogonalise(Integrator &I, int nv, double *w) {
-  bool normed = false;
+// Gram-Schmidt of w against V[0..nv): two classical passes (CGS2).  The
+// coefficients (of both passes) and |w|^2 come to the host: res()[0..nv], after wait().
+void orthogonalise(Integrator &I, int nv, double *w) {
+  const int n = I.n, g = red_blocks(n);
+  auto chunk = [&](int k0, VecPtrs &vp) {
+    const int cnt = std::min(kRedMax, nv - k0);
+    for (int k = 0; k < cnt; ++k) vp.v[k] = I.V[k0 + k];
+    return cnt;
+  };
+  VecPtrs vp;
+  if (nv <= kRedMax) {   // three launches
+    chunk(0, vp);
+    with_nvm(nv, [&](auto m) {
+      k_mdot<m(), false><<<g, 256, 0, I.s()>>>(n, nv, vp, w, I.hdev, I.hcol, 1, I.red(false));
+      k_mdot<m(), true><<<g, 256, 0, I.s()>>>(n, nv, vp, w, I.hdev, I.hcol, 0, I.red(false));
+      k_orth_norm<m()><<<g, 256, 0, I.s()>>>(n, nv, vp, I.hdev, w, nv, I.hcol, I.red());
+    });
+    I.hd->launches += 3;
+    return;
+  }
   for (int pass = 0; pass < 2; ++pass) {
-    for (int k0 = 0; k0 < nv; k0 += 32) {
-      int cnt = nv - k0 < 32 ? nv - k0 : 32;
-      VecPtrs vp;
-      for (int k = 0; k < cnt; ++k) vp.v[k] = I.V[k0 + k];
-      if (cnt <= 1) k_mdot<1><<<kRedBlocks, 256, 0, I.s()>>>(I.n, cnt, vp, w, I.part);
-      else if (cnt <= 2) k_mdot<2><<<kRedBlocks, 256, 0, I.s()>>>(I.n, cnt, vp, w, I.part);
-      else if (cnt <= 4) k_mdot<4><<<kRedBlocks, 256, 0, I.s()>>>(I.n, cnt, vp, w, I.part);
-      else if (cnt <= 8) k_mdot<8><<<kRedBlocks, 256, 0, I.s()>>>(I.n, cnt, vp, w, I.part);
-      else if (cnt <= 16) k_mdot<16><<<kRedBlocks, 256, 0, I.s()>>>(I.n, cnt, vp, w, I.part);
-      else k_mdot<32><<<kRedBlocks, 256, 0, I.s()>>>(I.n, cnt, vp, w, I.part);
-      ++I.hd->launches;
-      k_mdot_final<<<1, 256, 0, I.s()>>>(kRedBlocks, cnt, I.part, I.hdev.p + k0, I.hcol.p + k0, pass == 0);
+    for (int k0 = 0; k0 < nv; k0 += kRedMax) {
+      const int cnt = chunk(k0, vp);
+      with_nvm(cnt, [&](auto m) {
+        k_mdot<m(), false><<<g, 256, 0, I.s()>>>(n, cnt, vp, w, I.hdev.p + k0, I.hcol.p + k0, pass == 0, I.red(false));
+      });
       ++I.hd->launches;
     }
-    for (int k0 = 0; k0 < nv; k0 += 32) {
-      int cnt = nv - k0 < 32 ? nv - k0 : 32;
-      VecPtrs vp;
-      for (int k = 0; k < cnt; ++k) vp.v[k] = I.V[k0 + k];
-      if (pass == 1 && nv <= 32) {
-        launch_orth_norm(I.n, cnt, vp, I.hdev.p + k0, w, I.part, I.s());
-        normed = true;
-      } else {
-        launch_orth(I.n, cnt, vp, I.hdev.p + k0, w, I.s());
-      }
+    for (int k0 = 0; k0 < nv; k0 += kRedMax) {
+      const int cnt = chunk(k0, vp);
+      with_nvm(cnt, [&](auto m) { k_orth<m()><<<nblk(n, 256), 256, 0, I.s()>>>(n, cnt, vp, I.hdev.p + k0, w); });
       ++I.hd->launches;
     }
   }
-  return normed;
+  k_orth_norm<1><<<g, 256, 0, I.s()>>>(n, 0, vp, I.hdev, w, nv, I.hcol, I.red()); ++I.hd->launches;
 }
 
-// SPGMR, left preconditioned, scaled by ewt; x = 0 initial guess.
+// SPGMR, left preconditioned, scaled by ewt, zero initial guess: rho is the
+// norm of the preconditioned residual V[0].  Leaves the solution's coefficients
+// in I.yg[0..*nli_out) (x = sum_k yg_k V_k / ewt).
 // 0 converged, 2 residual reduced, 1 failure, <0 device error.
-int spgmr(Integrator &I, const double *b, double *x, double delta, int *nli_out) {
+int spgmr(Integrator &I, double rho, double delta, int *nli_out) {
   const int n = I.n, maxl = I.maxl;
   const Mesh &M = I.hd->mesh;
-  const nmg_material &mt = I.hd->mat;
   auto HM = [&](int i, int j) -> double & { return I.Hm[(size_t)i * maxl + j]; };
   *nli_out = 0;
-  k_psolve<<<nblk((long long)M.N * I.hd->nrep, 128), 128, 0, I.s()>>>((long long)n, I.Pinv, b, I.ewt, I.V[0]);
-  ++I.hd->launches;
-  I.nps++;
-  double rho = 0.0;  // ||V0||_2 (unweighted)
-  {
-    k_red<<<kRedBlocks, 256, 0, I.s()>>>(n, 1, I.V[0], I.V[0], I.part); ++I.hd->launches;
-    cudaMemcpyAsync(I.hpin, I.part.p, sizeof(double) * kRedBlocks, cudaMemcpyDeviceToHost, I.s());
-    if (cudaStreamSynchronize(I.s()) != cudaSuccess) return -1;
-    double acc = 0.0;
-    for (int bb = 0; bb < kRedBlocks; ++bb) acc += I.hpin[bb];
-    rho = std::sqrt(acc);
-  }
-  cudaMemsetAsync(x, 0, sizeof(double) * n, I.s());
   if (rho <= delta) return 0;
   I.beta0 = rho;
-  k_scale<<<nblk(n, 256), 256, 0, I.s()>>>(n, 1.0 / rho, I.V[0]); ++I.hd->launches;
+  double scale = 1.0 / rho;
   std::fill(I.yg.begin(), I.yg.end(), 0.0);
   I.yg[0] = rho;
   int converged = 0, kdim = 0;
   for (int l = 0; l < maxl; ++l) {
-    // t = V_l / ewt in its own pass: inside the FP64-bound Jv kernel the
-    // division would be repeated for every neighbour reference
-    if (jv_fp32(I.hd)) {
-      if (!I.K32.p) return -1;   // set up with every preconditioner setup (never reached)
-      k_div_ewt32<<<nblk(n, 256), 256, 0, I.s()>>>(n, I.V[l], I.ewts, I.t32); ++I.hd->launches;
+    const bool f32 = jv_fp32(I.hd);
+    if (f32 && !I.K32.p) return -1;   // set up with every preconditioner setup (never reached)
+    k_scale_dir<<<nblk(n, 256), 256, 0, I.s()>>>(n, scale, I.V[l], I.ewts, I.tvec, f32 ? I.t32.p : nullptr);
+    ++I.hd->launches;
+    if (f32) {
       Jv32Args a = jv32_base(I.hd);
       a.K = I.K32; a.mJ = I.mJ32; a.HJ = I.HJ32; a.t = I.t32; a.Pinv = I.Pinv32; a.ewt = I.ewt;
       a.gamma = I.gamma; a.psolve = 1; a.scale_out = 1; a.out = I.V[l + 1];
@@ -844,7 +917,6 @@ int spgmr(Integrator &I, const double *b, double *x, double delta, int *nli_out)
       ++I.hd->launches;
       NMG_PROF_END(I.hd);
     } else {
-      k_div_ewt<<<nblk(n, 256), 256, 0, I.s()>>>(n, I.V[l], I.ewts, I.tvec); ++I.hd->launches;
       JvArgs a = jv_args(I, I.tvec, I.V[l + 1], 1);
       if (demag_in_jacobian(I.hd)) {   // exact Jacobian: the demag field of the direction
         if (demag_response(I.hd, I.tvec)) return -1;
@@ -857,18 +929,10 @@ int spgmr(Integrator &I, const double *b, double *x, double delta, int *nli_out)
       NMG_PROF_END(I.hd);
     }
     I.njv++; I.nps++;
-    if (!orthogonalise(I, l + 1, I.V[l + 1])) {
-      k_red<<<kRedBlocks, 256, 0, I.s()>>>(n, 1, I.V[l + 1], I.V[l + 1], I.part);
-      ++I.hd->launches;
-    }
-    cudaMemcpyAsync(I.hpin, I.hcol.p, sizeof(double) * (l + 1), cudaMemcpyDeviceToHost, I.s());
-    double *hp2 = I.hpin + maxl + 1;
-    cudaMemcpyAsync(hp2, I.part.p, sizeof(double) * kRedBlocks, cudaMemcpyDeviceToHost, I.s());
-    if (cudaStreamSynchronize(I.s()) != cudaSuccess) return -1;
-    for (int k = 0; k <= l; ++k) HM(k, l) = I.hpin[k];
-    double acc = 0.0;
-    for (int bb = 0; bb < kRedBlocks; ++bb) acc += hp2[bb];
-    double hn = std::sqrt(acc);
+    orthogonalise(I, l + 1, I.V[l + 1]);
+    if (!I.wait()) return -1;
+    for (int k = 0; k <= l; ++k) HM(k, l) = I.res()[k];
+    double hn = std::sqrt(I.res()[l + 1]);
     HM(l + 1, l) = hn;
     for (int k = 0; k < l; ++k) {
       double c = I.gv[2 * k], sn = I.gv[2 * k + 1];
@@ -889,7 +953,7 @@ int spgmr(Integrator &I, const double *b, double *x, double delta, int *nli_out)
     kdim = l + 1;
     if (rho <= delta) { converged = 1; break; }
     if (hn == 0.0) break;
-    k_scale<<<nblk(n, 256), 256, 0, I.s()>>>(n, 1.0 / hn, I.V[l + 1]); ++I.hd->launches;
+    scale = 1.0 / hn;
   }
   *nli_out = kdim;
   for (int k = kdim - 1; k >= 0; --k) {
@@ -897,30 +961,56 @@ int spgmr(Integrator &I, const double *b, double *x, double delta, int *nli_out)
     for (int j = k + 1; j < kdim; ++j) sum -= HM(k, j) * I.yg[j];
     I.yg[k] = sum / HM(k, k);
   }
-  for (int k0 = 0; k0 < kdim; k0 += 32) {
-    int cnt = kdim - k0 < 32 ? kdim - k0 : 32;
-    VecPtrs vp;
-    for (int k = 0; k < cnt; ++k) vp.v[k] = I.V[k0 + k];
-    Coef32 c;
-    for (int k = 0; k < cnt; ++k) c.c[k] = I.yg[k0 + k];
-    launch_axpy_multi(n, cnt, vp, c, x, I.s());   // x -= (-y) V, as the Gram-Schmidt update
-    ++I.hd->launches;
-  }
-  k_div_ewt<<<nblk(n, 256), 256, 0, I.s()>>>(n, x, I.ewts, x); ++I.hd->launches;
   if (converged) return 0;
   return (rho < I.beta0) ? 2 : 1;
 }
 
+// acor += b, y = zn0 + acor with b = sum_k yg_k V_k / ewt (kdim >= 0) or the
+// Newton residual itself (kdim < 0); returns the WRMS norm of b.
+double newton_end(Integrator &I, int kdim) {
+  const int n = I.n, res = kdim < 0 ? 1 : 0;
+  const double *x0 = res ? I.tempv.p : nullptr;
+  VecPtrs vp;
+  Coef32 c;
+  auto chunk = [&](int k0) {
+    const int cnt = std::max(0, std::min(kRedMax, kdim - k0));
+    for (int k = 0; k < cnt; ++k) { vp.v[k] = I.V[k0 + k]; c.c[k] = I.yg[k0 + k]; }
+    return cnt;
+  };
+  int k0 = 0;
+  if (kdim > kRedMax) {   // all but the last vectors first
+    cudaMemsetAsync(I.xsol.p, 0, sizeof(double) * n, I.s());
+    for (; kdim - k0 > kRedMax; k0 += kRedMax) {
+      const int cnt = chunk(k0);
+      k_axpy_multi<kRedMax><<<nblk(n, 256), 256, 0, I.s()>>>(n, cnt, vp, c, I.xsol); ++I.hd->launches;
+    }
+    x0 = I.xsol.p;
+  }
+  const int cnt = chunk(k0);
+  with_nvm(cnt, [&](auto m) {
+    k_newton_end<m()><<<red_blocks(n), 256, 0, I.s()>>>(n, cnt, vp, c, x0, res, I.ewt, I.ewts, I.zn[0], I.acor, I.y,
+                                                       I.red());
+  });
+  ++I.hd->launches;
+  if (!I.wait()) { I.status = 100; return 0.0; }
+  return std::sqrt(I.res()[0] / n);
+}
+
 void predict(Integrator &I) {
   I.tn += I.h;
-  NMG_LAUNCH_Q(k_predict, I.q, nblk(I.n, 256), 256, I.s(), I.n, I.znp(), 1); ++I.hd->launches;
+  NMG_LAUNCH_Q(k_predict, I.q, nblk(I.n, 256), 256, I.s(), I.n, I.znp(), 1, I.eta_due, I.rtol, I.atol,
+               I.ewt_due ? I.ewt.p : nullptr, I.ewts.p); ++I.hd->launches;
+  I.eta_due = 1.0;
+  I.ewt_due = false;
 }
 void restore(Integrator &I, double saved_t) {
   I.tn = saved_t;
-  NMG_LAUNCH_Q(k_predict, I.q, nblk(I.n, 256), 256, I.s(), I.n, I.znp(), -1); ++I.hd->launches;
+  NMG_LAUNCH_Q(k_predict, I.q, nblk(I.n, 256), 256, I.s(), I.n, I.znp(), -1, 1.0, I.rtol, I.atol,
+               static_cast<double *>(nullptr), I.ewts.p); ++I.hd->launches;
 }
+// The history takes the new step with the prediction, which always follows.
 void rescale(Integrator &I) {
-  NMG_LAUNCH_Q(k_rescale, I.q, nblk(I.n, 256), 256, I.s(), I.n, I.znp(), I.eta); ++I.hd->launches;
+  I.eta_due = I.eta;
   I.h = I.hscale * I.eta;
   I.hprime = I.h;
   I.hscale = I.h;
@@ -1017,33 +1107,32 @@ int nls(Integrator &I, int nflag_first) {
         ++I.hd->launches;
       }
     }
-    cudaMemsetAsync(I.acor.p, 0, sizeof(double) * n, I.s());
-    cudaMemcpyAsync(I.y.p, I.zn[0], sizeof(double) * n, cudaMemcpyDeviceToDevice, I.s());
     int m = 0, retry = 0;
     double delp = 0.0, del;
     for (;;) {
       I.nni++;
-      k_newton_res<<<nblk(n, 256), 256, 0, I.s()>>>(n, I.gamma, I.ftemp, I.rl1, I.zn[1], I.acor, I.tempv); ++I.hd->launches;
+      const int nodes = n / 3;
+      k_newton_start<<<red_blocks(nodes), 256, 0, I.s()>>>(nodes, m == 0, I.gamma, I.ftemp, I.rl1, I.zn[0], I.zn[1],
+                                                          I.acor, I.y, I.Pinv, I.ewt, I.tempv, I.V[0], I.red());
+      ++I.hd->launches;
       double deltar = SPILS_DELT * I.tq[4];
-      double bnorm = I.wrms(I.tempv, I.ewt);
-      if (I.status) return -4;
-      int lflag = 0;
-      if (bnorm <= deltar) {
-        if (m > 0) cudaMemsetAsync(I.tempv.p, 0, sizeof(double) * n, I.s());
-      } else {
-        int nli = 0;
-        int sr = spgmr(I, I.tempv, I.xsol, deltar * std::sqrt((double)n), &nli);
+      if (!I.wait()) { I.status = 100; return -4; }
+      double bnorm = std::sqrt(I.res()[0] / n);
+      const double rho = std::sqrt(I.res()[1]);   // of the preconditioned residual
+      int lflag = 0, kdim = m > 0 ? 0 : -1;
+      if (!(bnorm <= deltar)) {
+        I.nps++;
+        int sr = spgmr(I, rho, deltar * std::sqrt((double)n), &kdim);
         if (sr < 0) return -4;
-        I.nli += nli;
-        cudaMemcpyAsync(I.tempv.p, I.xsol.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, I.s());
+        I.nli += kdim;
         if (sr == 1 || (sr == 2 && m > 0)) lflag = 1;
       }
       if (lflag) {
         if (!I.jcur) { convfail_bad_j = 1; call_setup = 1; retry = 1; }
         break;
       }
-      del = I.wrms(I.tempv, I.ewt);
-      k_newton_upd<<<nblk(n, 256), 256, 0, I.s()>>>(n, I.tempv, I.acor, I.zn[0], I.y); ++I.hd->launches;
+      del = newton_end(I, kdim);
+      if (I.status) return -4;
       if (m > 0) { double r = del / delp; I.crate = CRDOWN * I.crate > r ? CRDOWN * I.crate : r; }
       double dcon = del * (I.crate < 1.0 ? I.crate : 1.0) / I.tq[4];
       if (dcon <= 1.0) {
@@ -1070,12 +1159,13 @@ void complete_step(Integrator &I) {
   I.tau[1] = I.h;
   Coef c;
   for (int j = 0; j < QMAXB + 2; ++j) c.c[j] = j <= QMAXB ? I.l[j] : 0.0;
-  NMG_LAUNCH_Q(k_complete, I.q, nblk(I.n, 256), 256, I.s(), I.n, I.znp(), c, I.acor); ++I.hd->launches;
   I.qwait--;
+  double *save = nullptr;
   if (I.qwait == 1 && I.q != I.qmax) {
-    cudaMemcpyAsync(I.zn[I.qmax], I.acor.p, sizeof(double) * I.n, cudaMemcpyDeviceToDevice, I.s());
+    save = I.zn[I.qmax];
     I.saved_tq5 = I.tq[5];
   }
+  NMG_LAUNCH_Q(k_complete, I.q, nblk(I.n, 256), 256, I.s(), I.n, I.znp(), c, I.acor.p, save); ++I.hd->launches;
 }
 
 void adjust_order(Integrator &I, int deltaq) {
@@ -1232,10 +1322,12 @@ Integrator *ts_create(nmg_handle *h, int qmax, int maxl, double rtol, double ato
     ok = ok && b->alloc(n) == cudaSuccess;
   ok = ok && I->Vbuf.alloc(n * (I->maxl + 1)) == cudaSuccess;
   ok = ok && I->Pinv.alloc(3 * n) == cudaSuccess;
-  ok = ok && I->part.alloc(32 * kRedBlocks) == cudaSuccess;
+  ok = ok && I->part.alloc(kRedMax * kRedBlocks) == cudaSuccess;
+  ok = ok && I->redcnt.alloc(1) == cudaSuccess && cudaMemset(I->redcnt.p, 0, sizeof(unsigned)) == cudaSuccess;
   ok = ok && I->hdev.alloc(I->maxl + 64) == cudaSuccess;
   ok = ok && I->hcol.alloc(I->maxl + 64) == cudaSuccess;
-  ok = ok && cudaMallocHost(&I->hpin, sizeof(double) * (I->maxl + 1 + kRedBlocks + 64)) == cudaSuccess;
+  ok = ok && cudaMallocHost(&I->hpin, sizeof(double) * (I->maxl + 64)) == cudaSuccess;
+  if (ok) std::memset(I->hpin, 0, sizeof(double) * (I->maxl + 64));
   if (!ok) { ts_destroy(I); return nullptr; }
   for (int j = 0; j < QMAXB + 2; ++j) I->zn[j] = j <= I->qmax + 1 ? I->znbuf.p + n * j : nullptr;
   I->V.resize(I->maxl + 1);
@@ -1267,6 +1359,7 @@ int ts_init(nmg_handle *h, double t0) {
   I.nstlp = I.nstlpre = 0;
   I.etamax = ETAMX1; I.h = 0.0; I.hprime = 0.0; I.nlscoef = CORTES;
   I.setup_done = 0; I.jcur = 0; I.status = 0; I.saved_tq5 = 0.0;
+  I.eta_due = 1.0; I.ewt_due = false;
   for (int i = 0; i < QMAXB + 2; ++i) I.tau[i] = 0.0;
   for (int i = 0; i < 6; ++i) I.tq[i] = 0.0;
   cudaMemcpyAsync(I.zn[0], h->ws.m.p, sizeof(double) * I.n, cudaMemcpyDeviceToDevice, I.s());
@@ -1300,7 +1393,7 @@ int ts_advance(nmg_handle *h, double tout, int exact_tstop, int64_t max_steps, d
       break;
     }
     if (exact_tstop && (I.tn + I.hprime - tout) * I.hprime > 0.0) I.hprime = (tout - I.tn) * (1.0 - 4.0 * UROUND);
-    I.set_ewt(I.zn[0]);
+    I.ewt_due = true;
     int r = step(I);
     if (r) {
       rc = r;
@@ -1344,10 +1437,7 @@ int rk4_device(nmg_handle *h, double *d_m, double dt, int nsteps) {
     k_lin<<<nblk(n, 256), 256, 0, s>>>(n, 1.0, d_m, dt, k3, y); ++h->launches;
     if (rhs_eval(h, y, k4)) return 100;
     // m += dt/6 (k1 + 2 k2 + 2 k3 + k4)
-    k_lin<<<nblk(n, 256), 256, 0, s>>>(n, 1.0, k1, 2.0, k2, y); ++h->launches;
-    k_lin<<<nblk(n, 256), 256, 0, s>>>(n, 1.0, y, 2.0, k3, y); ++h->launches;
-    k_lin<<<nblk(n, 256), 256, 0, s>>>(n, 1.0, y, 1.0, k4, y); ++h->launches;
-    k_lin<<<nblk(n, 256), 256, 0, s>>>(n, 1.0, d_m, dt / 6.0, y, d_m); ++h->launches;
+    k_rk4<<<nblk(n, 256), 256, 0, s>>>(n, dt / 6.0, k1, k2, k3, k4, d_m); ++h->launches;
   }
   return check_device_error(h, "rk4");
 }
