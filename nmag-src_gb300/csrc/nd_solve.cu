@@ -425,6 +425,8 @@ struct NdArgs {
   const double *b;
   const double *one, *kone;   // mode 0: the sweeps' answer to b = 1 and K times it (null: sweeps alone, x as they give it)
   double *x, *xw, *r, *part;
+  NdOut out;
+  int nbnd;
   void *u, *d;
   unsigned *bar;
   int *err, *iters;
@@ -597,7 +599,11 @@ __global__ void __launch_bounds__(kNdThreads, 1) k_nd_solve(NdArgs a) {
         const double t = m < a.nm ? a.b[(size_t)m * a.N + i] : 0.0;
         v[w] += t;
         v[MW + w] += t * t;
-        if (fixed && m < a.nm) a.x[(size_t)m * a.N + i] = t;
+        if (fixed && m < a.nm) {
+          const size_t o = (size_t)m * a.N + i;
+          a.x[o] = t;
+          if (a.out.sum) a.out.sum[o] = a.out.add[o] + t;
+        }
       }
     }
     nd_partial<MB, MW>(v, s_sm, slot0);
@@ -828,7 +834,13 @@ __global__ void __launch_bounds__(kNdThreads, 1) k_nd_solve(NdArgs a) {
         if (m >= a.nm) continue;
         double t = __ldcg(a.xw + (size_t)p * MB + m);
         if (a.one) t = (t - s_mean[m] * w1) - s_res[MB + m] / a.N;   // mode 0
-        a.x[(size_t)m * a.N + i] = t;
+        const size_t o = (size_t)m * a.N + i;
+        a.x[o] = t;
+        if (a.out.sum) a.out.sum[o] = a.out.add[o] + t;
+        if (a.out.bnd) {
+          const int bi = a.b_of_node[i];
+          if (bi >= 0) a.out.bnd[(size_t)m * a.nbnd + bi] = t;
+        }
       }
     }
   }
@@ -1245,7 +1257,8 @@ void nd_reset_barrier(nmg_handle *h) {
   if (h->nd.bar.p) cudaMemsetAsync(h->nd.bar.p, 0, 2 * sizeof(unsigned), h->stream);
 }
 
-int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32) {
+int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32,
+             const NdOut &out) {
   NdSolver &D = h->nd;
   NdSystem &S = D.sys[mode];
   Workspace &W = h->ws;
@@ -1255,6 +1268,7 @@ int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double
   a.bnd = S.bnd; a.map = S.map; a.perm = S.perm; a.prow = S.prow; a.pcol = S.pcol; a.b_of_node = h->mesh.b_of_node;
   a.pK = S.pK;
   a.fac = fp32 ? (const void *)S.f32.p : (const void *)S.f64.p;
+  a.out = out; a.nbnd = h->mesh.nb;
   a.b = b; a.x = x; a.xw = D.xw; a.r = D.r; a.part = D.part; a.u = D.u.p; a.d = D.d.p;
   a.bar = D.bar; a.err = W.err; a.iters = W.iters;
   a.one = mode == 0 ? S.one.p : nullptr;

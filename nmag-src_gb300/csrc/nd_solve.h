@@ -22,4 +22,12 @@ struct NdFront {    // a part of the separator tree eliminated together
 struct NdTask { int front, start, count; };      // rows of a front (upwards: of its nb, downwards: of its k)
 struct NdLevel { int t0, t1, cs, pad; };         // one phase of a sweep: its tasks, warps sharing a row
 
+// What the next kernels of the demag pipeline read, written with the answer
+// (all may be null): its values at the boundary nodes, and sum = add + x.
+struct NdOut {
+  double *bnd = nullptr;
+  const double *add = nullptr;
+  double *sum = nullptr;
+};
+
 }  // namespace nmg

@@ -332,6 +332,29 @@ struct nmg_handle {
   if (prof_slot__ >= 0) (h)->prof.end((h)->stream, prof_slot__)
 
 namespace nmg {
+// Sum over the L neighbouring lanes that share a matrix row (each gets it).
+template <int L>
+__device__ __forceinline__ double lane_sum(double v) {
+  const unsigned mask = (L == 32 ? 0xffffffffu : (1u << (L & 31)) - 1u) << (threadIdx.x & 31 & ~(L - 1));
+#pragma unroll
+  for (int o = L / 2; o; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+  return v;
+}
+// Up to this many nodes four lanes share a row, in one-warp blocks: with a row
+// per thread the cube's 1,331 rows are 42 warps, and in blocks of 128 they sat on
+// 11 SMs whose FP64 pipes they shared (k_heff_llg 12.0 -> 9.8 us, k_div 9.1 ->
+// 5.8, k_dbc_rhs 9.4 -> 4.5).  Larger meshes fill the chip with a row per thread,
+// and the lane sums' FP64 adds would cost more than they hide (film, 30,753
+// rows: k_heff_llg 16 against 27 us).
+constexpr int kRowLanesMax = 8192;
+// Launch K<lanes>(...) over `rows` matrix rows of a mesh of N nodes.
+#define NMG_LAUNCH_ROWS(K, N, rows, st, ...)                                                            \
+  do {                                                                                                  \
+    if ((N) <= nmg::kRowLanesMax)                                                                       \
+      K<4><<<(unsigned)((4 * (long long)(rows) + 31) / 32), 32, 0, st>>>(__VA_ARGS__);                  \
+    else                                                                                                \
+      K<1><<<(unsigned)(((long long)(rows) + 63) / 64), 64, 0, st>>>(__VA_ARGS__);                      \
+  } while (0)
 // Compensated FP32 multiply-add of the BEM products: (S, C) += (h + l)(a + b)
 // with h*a split exactly by an FMA, the second-order terms h*b + l*a added to
 // the error term, and S updated by TwoSum (~44 bits in FP32 operations).
@@ -377,7 +400,8 @@ int jac_demag_solve(nmg_handle *P, JacDemag &J, double rtol);
 // to max(rtol |b|, atol).
 int nd_prepare(nmg_handle *h);
 bool nd_available(const nmg_handle *h, int mode);
-int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32);
+int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32,
+             const NdOut &out = NdOut());
 void nd_reset_barrier(nmg_handle *h);   // after a launch whose barrier gave up
 // ---- bem_tc.cu ----
 int bem_tc_setup(nmg_handle *h, std::string &err);

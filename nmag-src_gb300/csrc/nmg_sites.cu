@@ -36,20 +36,22 @@ namespace {
 inline unsigned nblk_s(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 // rho_s = -Ms_X (D m)_s on the site mesh (D is block diagonal by material).
+template <int L>
 __global__ void k_div_sites(int S, int nnz, const SiteMat *__restrict__ mt, const int32_t *__restrict__ site_mat,
                             const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col_idx,
                             const double *__restrict__ D, const double *__restrict__ m, double *__restrict__ rho,
                             int nrep) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / L;
   if (g >= (long long)S * nrep) return;
   const int b = (int)(g / S), s = (int)(g - (long long)b * S);
   const double *mb = m + (size_t)b * 3 * S;
   double acc = 0.0;
-  for (int k = row_ptr[s]; k < row_ptr[s + 1]; ++k) {
+  for (int k = row_ptr[s] + threadIdx.x % L, end = row_ptr[s + 1]; k < end; k += L) {
     const double *mj = mb + 3 * (size_t)col_idx[k];
     acc += (D[k] * mj[0] + D[(size_t)nnz + k] * mj[1]) + D[2 * (size_t)nnz + k] * mj[2];
   }
-  rho[g] = -(mt[site_mat[s]].Ms * acc);
+  acc = lane_sum<L>(acc);
+  if (threadIdx.x % L == 0) rho[g] = -(mt[site_mat[s]].Ms * acc);
 }
 
 // rho_i (potential mesh) = sum over the sites of node i, in site order.
@@ -101,30 +103,34 @@ __device__ __forceinline__ void local_coupling(const SiteArgs &a, int s, int X, 
   }
 }
 
+template <int L>
 __global__ void k_heff_llg_sites(SiteArgs a) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / L;
   if (g >= (long long)a.S * a.nrep) return;
   const int b = (int)(g / a.S), s = (int)(g - (long long)b * a.S);
   const SiteMat c = a.mt[a.site_mat[s]];
   const double *mm = a.m + (size_t)b * 3 * a.S;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-  for (int k = a.row_ptr[s]; k < a.row_ptr[s + 1]; ++k) {
+  for (int k = a.row_ptr[s] + threadIdx.x % L, end = a.row_ptr[s + 1]; k < end; k += L) {
     const double *mj = mm + 3 * (size_t)a.col_idx[k];
     const double kv = a.K[k];
     s0 += kv * mj[0]; s1 += kv * mj[1]; s2 += kv * mj[2];
   }
+  s0 = lane_sum<L>(s0); s1 = lane_sum<L>(s1); s2 = lane_sum<L>(s2);
   double hd[3] = {0.0, 0.0, 0.0};
   if (a.phi) {
     const int i = a.site_node[s];
     const double *ph = a.phi + (size_t)b * a.Np;
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    for (int k = a.prow[i]; k < a.prow[i + 1]; ++k) {
+    for (int k = a.prow[i] + threadIdx.x % L, end = a.prow[i + 1]; k < end; k += L) {
       const double pj = ph[a.pcol[k]];
       g0 += a.G[k] * pj; g1 += a.G[(size_t)a.nnzp + k] * pj; g2 += a.G[2 * (size_t)a.nnzp + k] * pj;
     }
+    g0 = lane_sum<L>(g0); g1 = lane_sum<L>(g1); g2 = lane_sum<L>(g2);
     const double piv = a.pivol[i];
     hd[0] = -g0 * piv; hd[1] = -g1 * piv; hd[2] = -g2 * piv;
   }
+  if (threadIdx.x % L) return;
   const double ce = -c.c_exch * a.ivol[s];
   const double hx[3] = {ce * s0, ce * s1, ce * s2};
   const double *m = mm + 3 * (size_t)s;
@@ -237,7 +243,7 @@ int rhs_eval_sites(nmg_handle *h, const double *d_m, double *d_dmdt) {
   const long long SB = (long long)S * B;
   const bool demag = h->opt.do_demag && P->mesh.nb > 0;
   if (demag) {
-    k_div_sites<<<nblk_s(SB, 256), 256, 0, st>>>(S, M.nnz, h->sites.mtab, h->sites.site_mat, M.row_ptr, M.col_idx,
+    NMG_LAUNCH_ROWS(k_div_sites, S, SB, st, S, M.nnz, h->sites.mtab, h->sites.site_mat, M.row_ptr, M.col_idx,
                                                   M.D, d_m, W.rho, B);
     k_scatter_sites<<<nblk_s((long long)P->mesh.N * B, 256), 256, 0, st>>>(
         P->mesh.N, h->sites.node_ptr, h->sites.node_sites, W.rho, P->ws.rho, S, B);
@@ -264,7 +270,7 @@ int rhs_eval_sites(nmg_handle *h, const double *d_m, double *d_dmdt) {
   a.dmdt = d_dmdt ? d_dmdt : W.dmdt.p;
   {
     NMG_PROF_BEGIN(h, 3);
-    k_heff_llg_sites<<<nblk_s(SB, 128), 128, 0, st>>>(a);
+    NMG_LAUNCH_ROWS(k_heff_llg_sites, S, SB, st, a);
     ++h->launches;
     NMG_PROF_END(h);
   }
@@ -285,7 +291,7 @@ int demag_response_sites(nmg_handle *h, const double *d_v) {
   }
   const int S = M.N, B = h->nrep;
   cudaStream_t st = h->stream;
-  k_div_sites<<<nblk_s((long long)S * B, 256), 256, 0, st>>>(S, M.nnz, h->sites.mtab, h->sites.site_mat, M.row_ptr,
+  NMG_LAUNCH_ROWS(k_div_sites, S, (long long)S * B, st, S, M.nnz, h->sites.mtab, h->sites.site_mat, M.row_ptr,
                                                               M.col_idx, M.D, d_v, h->ws.rho, B);
   k_scatter_sites<<<nblk_s((long long)P->mesh.N * B, 256), 256, 0, st>>>(P->mesh.N, h->sites.node_ptr,
                                                                           h->sites.node_sites, h->ws.rho, J.rho, S, B);

@@ -501,18 +501,19 @@ __device__ __forceinline__ void jac_apply(const T *m, const T *H, const T *w, co
 
 // kLocal: Jacobian level >= 1 (local terms, demag response); the default
 // level 0 keeps the lean exchange-only form
-template <bool kLocal>
+template <bool kLocal, int L>
 __global__ void k_jv_psolve(JvArgs a) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / L;
   if (g >= (long long)a.N * a.nrep) return;
   const int mbr = (int)(g / a.N), i = (int)(g - (long long)mbr * a.N);
   const double *tm = a.t + (size_t)mbr * 3 * a.N;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-  for (int k = a.row_ptr[i]; k < a.row_ptr[i + 1]; ++k) {
+  for (int k = a.row_ptr[i] + threadIdx.x % L, end = a.row_ptr[i + 1]; k < end; k += L) {
     const double *tj = tm + 3 * (size_t)a.col_idx[k];
     double kv = a.K[k];
     s0 += kv * tj[0]; s1 += kv * tj[1]; s2 += kv * tj[2];
   }
+  s0 = lane_sum<L>(s0); s1 = lane_sum<L>(s1); s2 = lane_sum<L>(s2);
   double c_exch = a.c_exch, C1 = a.C1, C2 = a.C2;
   if (a.site_mat) {
     const SiteMat &c = a.mt[a.site_mat[i]];
@@ -530,6 +531,7 @@ __global__ void k_jv_psolve(JvArgs a) {
       hv[0] += q[0]; hv[1] += q[1]; hv[2] += q[2];
     }
   }
+  if (threadIdx.x % L) return;
   double jw[3];
   jac_apply(m, H, w, hv, C1, C2, jw);
   if constexpr (kLocal) {
@@ -851,6 +853,14 @@ JvArgs jv_args(Integrator &I, const double *t, double *out, int psolve) {
   return a;
 }
 
+template <int L> constexpr auto k_jv_local = k_jv_psolve<true, L>;
+template <int L> constexpr auto k_jv_plain = k_jv_psolve<false, L>;
+void launch_jv_psolve(const nmg_handle *h, const JvArgs &a) {
+  const long long rows = (long long)a.N * a.nrep;
+  if (a.L.on) NMG_LAUNCH_ROWS(k_jv_local, a.N, rows, h->stream, a);
+  else NMG_LAUNCH_ROWS(k_jv_plain, a.N, rows, h->stream, a);
+}
+
 // Gram-Schmidt of w against V[0..nv): two classical passes (CGS2).  The
 // coefficients (of both passes) and |w|^2 come to the host: res()[0..nv], after wait().
 void orthogonalise(Integrator &I, int nv, double *w) {
@@ -923,8 +933,7 @@ int spgmr(Integrator &I, double rho, double delta, int *nli_out) {
         a.hdv = I.hd->jd.hdv;
       }
       NMG_PROF_BEGIN(I.hd, 4);
-      if (a.L.on) k_jv_psolve<true><<<nblk((long long)M.N * I.hd->nrep, 128), 128, 0, I.s()>>>(a);
-      else k_jv_psolve<false><<<nblk((long long)M.N * I.hd->nrep, 128), 128, 0, I.s()>>>(a);
+      launch_jv_psolve(I.hd, a);
       ++I.hd->launches;
       NMG_PROF_END(I.hd);
     }
@@ -1469,8 +1478,7 @@ int jacobian_apply(nmg_handle *h, const double *d_m, const double *d_v, double *
     if (demag_response(h, d_v)) return 100;
     a.hdv = h->jd.hdv;
   }
-  if (a.L.on) k_jv_psolve<true><<<nblk((long long)h->mesh.N * h->nrep, 128), 128, 0, h->stream>>>(a);
-  else k_jv_psolve<false><<<nblk((long long)h->mesh.N * h->nrep, 128), 128, 0, h->stream>>>(a);
+  launch_jv_psolve(h, a);
   ++h->launches;
   if (cudaGetLastError() != cudaSuccess) return 100;
   return check_device_error(h, "nmg_jacobian_apply");

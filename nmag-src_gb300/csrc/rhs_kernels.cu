@@ -1438,19 +1438,21 @@ __global__ void k_dinv(int N, const int32_t *__restrict__ diag_pos, const double
 }
 
 // rho = -(Ms * sum_k (D_x m_x + D_y m_y + D_z m_z))
+template <int L>
 __global__ void k_div(int N, int nnz, double Ms, const int32_t *__restrict__ row_ptr,
                       const int32_t *__restrict__ col_idx, const double *__restrict__ D,
                       const double *__restrict__ m, double *__restrict__ rho, int nrep = 1) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / L;
   if (g >= (long long)N * nrep) return;
   const int b = (int)(g / N), i = (int)(g - (long long)b * N);
   const double *mb = m + (size_t)b * 3 * N;
   double s = 0.0;
-  for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k) {
+  for (int k = row_ptr[i] + threadIdx.x % L, end = row_ptr[i + 1]; k < end; k += L) {
     const double *mj = mb + 3 * (size_t)col_idx[k];
     s += (D[k] * mj[0] + D[(size_t)nnz + k] * mj[1]) + D[2 * (size_t)nnz + k] * mj[2];
   }
-  rho[g] = -(Ms * s);
+  s = lane_sum<L>(s);
+  if (threadIdx.x % L == 0) rho[g] = -(Ms * s);
 }
 
 __global__ void k_gather_b(int nb, const int32_t *__restrict__ node_of_b, const double *__restrict__ phi,
@@ -1571,6 +1573,25 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemv_f32(int nb, int ld, long 
 }
 
 // y[r] = sum of the partials of the warps whose unit range meets row r, in
+// y = B x for a boundary of fewer rows than k_gemv_f64 has segments, where that
+// splits every row: a block of four warps per row, and no partials to add up in
+// another launch (602 nodes: 11.4 us of two kernels -> 4.4).
+__global__ void __launch_bounds__(128) k_gemv_f64_rows(int nb, int ld, const double *__restrict__ B,
+                                                       const double *__restrict__ x, double *__restrict__ y) {
+  __shared__ double sm[4];
+  const double *row = B + blockIdx.x * (size_t)ld;
+  double acc0 = 0.0, acc1 = 0.0;
+#pragma unroll 4
+  for (int c = 2 * threadIdx.x; c < ld; c += 256) {   // (ld is even; past nb: entries 0)
+    const double2 v = __ldcs(reinterpret_cast<const double2 *>(row + c));
+    acc0 = fma(v.x, __ldg(x + min(c, nb - 1)), acc0);
+    acc1 = fma(v.y, __ldg(x + min(c + 1, nb - 1)), acc1);
+  }
+  const double s = warp_sum(acc0 + acc1);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) y[blockIdx.x] = (sm[0] + sm[1]) + (sm[2] + sm[3]);
+}
 // warp order (Q = units per row).
 __global__ void k_row_sum(int nb, long long Q, long long seg, int maxr, long long nwarps,
                           const double *__restrict__ part, double *__restrict__ y) {
@@ -2119,22 +2140,24 @@ __global__ void k_anchor_row_sum(int nb, long long Q, long long seg, int maxr, l
 // Dirichlet right-hand side (op_load_DBC, sign folded): interior rows
 // -sum_{j boundary} K_ij phi2b_j, boundary rows phi2b; boundary values of the
 // warm start are set to phi2b.
+template <int L>
 __global__ void k_dbc_rhs(int N, const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col_idx,
                           const double *__restrict__ K, const int32_t *__restrict__ b_of_node,
                           const double *__restrict__ phi2b_all, double *__restrict__ rhs, double *__restrict__ phi2,
-                          int nb = 0, int nrep = 1) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+                          int nb, int nrep) {
+  const long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / L;
   if (g >= (long long)N * nrep) return;
   const int mbr = (int)(g / N), i = (int)(g - (long long)mbr * N);
   const double *phi2b = phi2b_all + (size_t)mbr * nb;
   int bi = b_of_node[i];
   if (bi >= 0) { rhs[g] = phi2b[bi]; phi2[g] = phi2b[bi]; return; }
   double s = 0.0;
-  for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k) {
+  for (int k = row_ptr[i] + threadIdx.x % L, end = row_ptr[i + 1]; k < end; k += L) {
     int b = b_of_node[col_idx[k]];
     if (b >= 0) s += K[k] * phi2b[b];
   }
-  rhs[g] = -s;
+  s = lane_sum<L>(s);
+  if (threadIdx.x % L == 0) rhs[g] = -s;
 }
 
 __global__ void k_add(int n, const double *__restrict__ a, const double *__restrict__ b, double *__restrict__ c) {
@@ -2201,15 +2224,16 @@ struct NodeArgs {
 };
 
 // Fused node kernel: the two SpMV epilogues and every site-wise equation.
+template <int L>
 __global__ void k_heff_llg(NodeArgs a) {
-  const long long gi = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long gi = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / L;
   if (gi >= (long long)a.N * a.nrep) return;
   const int mbr = (int)(gi / a.N), i = (int)(gi - (long long)mbr * a.N);
   const double *mm = a.m + (size_t)mbr * 3 * a.N;
   const double *ph = a.do_demag ? a.phi + (size_t)mbr * a.N : a.phi;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, g0 = 0.0, g1 = 0.0, g2 = 0.0;
   const int lo = a.row_ptr[i], hi = a.row_ptr[i + 1];
-  for (int k = lo; k < hi; ++k) {
+  for (int k = lo + threadIdx.x % L; k < hi; k += L) {
     const int j = a.col_idx[k];
     const double kv = a.K[k];
     const double *mj = mm + 3 * (size_t)j;
@@ -2219,6 +2243,8 @@ __global__ void k_heff_llg(NodeArgs a) {
       g0 += a.G[k] * pj; g1 += a.G[(size_t)a.nnz + k] * pj; g2 += a.G[2 * (size_t)a.nnz + k] * pj;
     }
   }
+  s0 = lane_sum<L>(s0); s1 = lane_sum<L>(s1); s2 = lane_sum<L>(s2);
+  if (a.do_demag) { g0 = lane_sum<L>(g0); g1 = lane_sum<L>(g1); g2 = lane_sum<L>(g2); }
   const double iv = a.ivol[i];
   const double ce = -a.c_exch * iv;
   const double hx[3] = {ce * s0, ce * s1, ce * s2};
@@ -2256,6 +2282,7 @@ __global__ void k_heff_llg(NodeArgs a) {
     const double p = a.pin[i];
     for (int d = 0; d < 3; ++d) f[d] *= p;
   }
+  if (threadIdx.x % L) return;
   for (int d = 0; d < 3; ++d) {
     const size_t o = 3 * (size_t)gi + d;
     a.h_exch[o] = hx[d]; a.h_demag[o] = hd[d]; a.h_anis[o] = ha[d]; a.h_total[o] = H[d];
@@ -2494,8 +2521,10 @@ void wait_basis_factor(nmg_handle *h, int ev_slot) {
     cudaStreamWaitEvent(h->stream, W.ev_ldl[ev_slot], 0);
 }
 
-int run_cg(nmg_handle *h, int mode, const double *b, double *x, double rtol, double atol, int maxits) {
-  if (nd_available(h, mode & 1)) return nd_solve(h, mode & 1, 1, b, x, rtol, atol, false);
+// `out` (the direct solves alone): what else is written with the answer.
+int run_cg(nmg_handle *h, int mode, const double *b, double *x, double rtol, double atol, int maxits,
+           const NdOut &out = NdOut()) {
+  if (nd_available(h, mode & 1)) return nd_solve(h, mode & 1, 1, b, x, rtol, atol, false, out);
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   CGArgs a;
@@ -2538,9 +2567,9 @@ int run_cg(nmg_handle *h, int mode, const double *b, double *x, double rtol, dou
 // bslot: warm-start basis slot of a single simulation (-1: `mode`); mp: 1
 // mixed precision, 0 FP64, -1 the handle's forward choice.
 int run_cgm(nmg_handle *h, int mode, int c0, const double *b, double *x, int nm, double rtol, double atol,
-            int maxits, int bslot = -1, int mp_sel = -1) {
+            int maxits, int bslot = -1, int mp_sel = -1, const NdOut &out = NdOut()) {
   if (nd_available(h, mode))
-    return nd_solve(h, mode, nm, b, x, rtol, atol, mp_sel >= 0 ? mp_sel == 1 : h->opt.cg_precision == 1);
+    return nd_solve(h, mode, nm, b, x, rtol, atol, mp_sel >= 0 ? mp_sel == 1 : h->opt.cg_precision == 1, out);
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   CGArgs a;
@@ -2867,6 +2896,11 @@ void bem_gemv(nmg_handle *h, const double *x, double *y) {
     NMG_PROF_BEGIN(h, 0);
     k_gemv_f32<<<W.gemv_blocks, kGemvThreads, 0, h->stream>>>(nb, M.ld, seg, maxr, M.bem32, x32, W.bpart); ++h->launches;
     NMG_PROF_END(h);
+  } else if (nb <= W.gemv_blocks * (kGemvThreads / 32)) {
+    NMG_PROF_BEGIN(h, 0);
+    k_gemv_f64_rows<<<nb, 128, 0, h->stream>>>(nb, M.ld, M.bem, x, y); ++h->launches;
+    NMG_PROF_END(h);
+    return;
   } else {
     NMG_PROF_BEGIN(h, 0);
     k_gemv_f64<<<W.gemv_blocks, kGemvThreads, 0, h->stream>>>(nb, M.ld, seg, maxr, M.bem, x, W.bpart); ++h->launches;
@@ -3086,30 +3120,41 @@ int demag_from_rho(nmg_handle *h) {
   cudaStream_t s = h->stream;
   const int N = M.N;
   const int B = h->nrep;
+  // the direct solves write the boundary values and phi1 + phi2 themselves
+  const bool nd0 = nd_available(h, 0), nd1 = nd_available(h, 1);
+  auto out = [&](int mode, int c0) {
+    NdOut o;
+    if (mode == 0) o.bnd = W.b1.p + (size_t)c0 * M.nb;
+    else { o.add = W.phi1.p + (size_t)c0 * N; o.sum = W.phi.p + (size_t)c0 * N; }
+    return o;
+  };
   if (B > 1) {
     // ensemble: the same pipeline over B members, kChunk members per CG / BEM launch
     const long long NB = (long long)N * B;
     for (int c0 = 0; c0 < B; c0 += kChunk)
       if (run_cgm(h, 0, c0, W.rho.p + (size_t)c0 * N, W.phi1.p + (size_t)c0 * N, std::min(kChunk, B - c0),
-                  h->opt.nbc_rtol, h->opt.nbc_atol, h->opt.nbc_maxits)) return 100;
-    k_gather_b<<<nblk((long long)M.nb * B, 256), 256, 0, s>>>(M.nb, M.node_of_b, W.phi1, W.b1, N, B); ++h->launches;
+                  h->opt.nbc_rtol, h->opt.nbc_atol, h->opt.nbc_maxits, -1, -1, out(0, c0))) return 100;
+    if (!nd0) {
+      k_gather_b<<<nblk((long long)M.nb * B, 256), 256, 0, s>>>(M.nb, M.node_of_b, W.phi1, W.b1, N, B); ++h->launches;
+    }
     bem_gemm(h, W.b1, W.b2);
-    k_dbc_rhs<<<nblk(NB, 256), 256, 0, s>>>(N, M.row_ptr, M.col_idx, M.K, M.b_of_node, W.b2, W.rhs2, W.phi2, M.nb, B);
+    NMG_LAUNCH_ROWS(k_dbc_rhs, N, NB, s, N, M.row_ptr, M.col_idx, M.K, M.b_of_node, W.b2, W.rhs2, W.phi2, M.nb, B);
     ++h->launches;
     for (int c0 = 0; c0 < B; c0 += kChunk)
       if (run_cgm(h, 1, c0, W.rhs2.p + (size_t)c0 * N, W.phi2.p + (size_t)c0 * N, std::min(kChunk, B - c0),
-                  h->opt.dbc_rtol, h->opt.dbc_atol, h->opt.dbc_maxits)) return 100;
-    k_add<<<nblk(NB, 256), 256, 0, s>>>((int)NB, W.phi1, W.phi2, W.phi); ++h->launches;
+                  h->opt.dbc_rtol, h->opt.dbc_atol, h->opt.dbc_maxits, -1, -1, out(1, c0))) return 100;
+    if (!nd1) { k_add<<<nblk(NB, 256), 256, 0, s>>>((int)NB, W.phi1, W.phi2, W.phi); ++h->launches; }
   } else {
     const bool mp = h->opt.cg_precision == 1;   // mixed-precision CG (one member)
-    if (mp ? run_cgm(h, 0, 0, W.rho, W.phi1, 1, h->opt.nbc_rtol, h->opt.nbc_atol, h->opt.nbc_maxits)
-           : run_cg(h, 0, W.rho, W.phi1, h->opt.nbc_rtol, h->opt.nbc_atol, h->opt.nbc_maxits)) return 100;
-    k_gather_b<<<nblk(M.nb, 256), 256, 0, s>>>(M.nb, M.node_of_b, W.phi1, W.b1); ++h->launches;
+    if (mp ? run_cgm(h, 0, 0, W.rho, W.phi1, 1, h->opt.nbc_rtol, h->opt.nbc_atol, h->opt.nbc_maxits, -1, -1, out(0, 0))
+           : run_cg(h, 0, W.rho, W.phi1, h->opt.nbc_rtol, h->opt.nbc_atol, h->opt.nbc_maxits, out(0, 0))) return 100;
+    if (!nd0) { k_gather_b<<<nblk(M.nb, 256), 256, 0, s>>>(M.nb, M.node_of_b, W.phi1, W.b1); ++h->launches; }
     bem_gemv(h, W.b1, W.b2);
-    k_dbc_rhs<<<nblk(N, 256), 256, 0, s>>>(N, M.row_ptr, M.col_idx, M.K, M.b_of_node, W.b2, W.rhs2, W.phi2); ++h->launches;
-    if (mp ? run_cgm(h, 1, 0, W.rhs2, W.phi2, 1, h->opt.dbc_rtol, h->opt.dbc_atol, h->opt.dbc_maxits)
-           : run_cg(h, 1, W.rhs2, W.phi2, h->opt.dbc_rtol, h->opt.dbc_atol, h->opt.dbc_maxits)) return 100;
-    k_add<<<nblk(N, 256), 256, 0, s>>>(N, W.phi1, W.phi2, W.phi); ++h->launches;
+    NMG_LAUNCH_ROWS(k_dbc_rhs, N, N, s, N, M.row_ptr, M.col_idx, M.K, M.b_of_node, W.b2, W.rhs2, W.phi2, M.nb, 1);
+    ++h->launches;
+    if (mp ? run_cgm(h, 1, 0, W.rhs2, W.phi2, 1, h->opt.dbc_rtol, h->opt.dbc_atol, h->opt.dbc_maxits, -1, -1, out(1, 0))
+           : run_cg(h, 1, W.rhs2, W.phi2, h->opt.dbc_rtol, h->opt.dbc_atol, h->opt.dbc_maxits, out(1, 0))) return 100;
+    if (!nd1) { k_add<<<nblk(N, 256), 256, 0, s>>>(N, W.phi1, W.phi2, W.phi); ++h->launches; }
   }
   return 0;
 }
@@ -3123,7 +3168,7 @@ int rhs_eval(nmg_handle *h, const double *d_m, double *d_dmdt) {
   const nmg_material &mt = h->mat;
   const int B = h->nrep;
   if (h->opt.do_demag && M.nb > 0) {
-    k_div<<<nblk((long long)N * B, 256), 256, 0, s>>>(N, M.nnz, mt.Ms, M.row_ptr, M.col_idx,
+    NMG_LAUNCH_ROWS(k_div, N, (long long)N * B, s, N, M.nnz, mt.Ms, M.row_ptr, M.col_idx,
                                                        h->ep.active ? h->ep.Dx.p : M.D.p, d_m, W.rho, B);
     ++h->launches;
     if (demag_from_rho(h)) return 100;
@@ -3154,7 +3199,7 @@ int rhs_eval(nmg_handle *h, const double *d_m, double *d_dmdt) {
   a.dmdt = d_dmdt ? d_dmdt : W.dmdt.p;
   {
     NMG_PROF_BEGIN(h, 3);
-    k_heff_llg<<<nblk((long long)N * B, 128), 128, 0, s>>>(a); ++h->launches;
+    NMG_LAUNCH_ROWS(k_heff_llg, N, (long long)N * B, s, a); ++h->launches;
     NMG_PROF_END(h);
   }
   h->n_rhs++;
@@ -3259,7 +3304,7 @@ int demag_response(nmg_handle *h, const double *d_v) {
     h->last_error = "exact Jacobian: cannot allocate the demag response buffers";
     return 100;
   }
-  k_div<<<nblk((long long)M.N * h->nrep, 256), 256, 0, h->stream>>>(M.N, M.nnz, h->mat.Ms, M.row_ptr, M.col_idx,
+  NMG_LAUNCH_ROWS(k_div, M.N, (long long)M.N * h->nrep, h->stream, M.N, M.nnz, h->mat.Ms, M.row_ptr, M.col_idx,
                                                                      h->ep.active ? h->ep.Dx.p : M.D.p, d_v, J.rho,
                                                                      h->nrep);
   ++h->launches;
