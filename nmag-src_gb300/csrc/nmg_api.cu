@@ -307,6 +307,8 @@ int nmg_eval_fields(nmg_handle *h, double *fields, double *scalars) {
   if (!h) return -1;
   int rc = nmg::rhs_eval(h, h->ws.m, h->ws.dmdt);
   if (rc) return fail(h, rc, "nmg_eval_fields: launch failed");
+  rc = nmg::post_fields(h, fields, scalars);
+  if (rc >= 0) return rc;
   rc = nmg::check_device_error(h, "nmg_eval_fields");
   if (rc) return rc;
   const size_t N = (size_t)h->mesh.N * h->nrep, n3 = 3 * N;

@@ -52,6 +52,47 @@ struct DevBuf {
   operator T *() const { return p; }
 };
 
+// Results that a kernel posts to the host: values from res() on, then the
+// sequence number, which the host waits for (a copy and a stream
+// synchronisation take ~15 us).  One post is under way at a time.
+struct HostPost {
+  double *buf = nullptr;   // pinned; the sequence number has the first line
+  size_t cap = 0;          // values
+  unsigned long long seq = 0;
+  HostPost() = default;
+  HostPost(const HostPost &) = delete;
+  HostPost &operator=(const HostPost &) = delete;
+  ~HostPost() {
+    if (buf) cudaFreeHost(buf);
+  }
+  bool reserve(size_t n) {   // with no post under way
+    if (n <= cap) return true;
+    if (buf) cudaFreeHost(buf);
+    buf = nullptr;
+    cap = 0;
+    seq = 0;
+    if (cudaMallocHost(&buf, sizeof(double) * (n + 8)) != cudaSuccess) {
+      buf = nullptr;
+      cudaGetLastError();
+      return false;
+    }
+    *flag() = 0;
+    cap = n;
+    return true;
+  }
+  double *res() const { return buf + 8; }
+  unsigned long long *flag() const { return reinterpret_cast<unsigned long long *>(buf); }
+  // Waits for the post numbered seq; false if its kernel did not run.
+  bool wait(cudaStream_t s) const {
+    for (unsigned spins = 1;; ++spins) {
+      if (__atomic_load_n(flag(), __ATOMIC_ACQUIRE) == seq) return true;
+      if (spins & 0xfff) continue;
+      const cudaError_t e = cudaStreamQuery(s);   // a launch that failed never posts
+      if (e != cudaErrorNotReady) return e == cudaSuccess && __atomic_load_n(flag(), __ATOMIC_ACQUIRE) == seq;
+    }
+  }
+};
+
 // Triangle geometry for the Lindholm evaluation (bem3d_stubs.c:466-525).
 struct TriGeo {
   double p[3][3], s_l[3], eta[3][3], zeta_v[3], gam01, gam12, gam20, factor, maxgeo;
@@ -291,6 +332,8 @@ struct nmg_handle {
   nmg::Integrator *ts = nullptr;
   int ts_ready = 0;             // integrator initialised for the current m / H_ext / material
   double *h_pinned = nullptr;   // small pinned staging buffer for scalars
+  nmg::HostPost post;                  // fields, averages and the like of small meshes
+  nmg::DevBuf<unsigned> post_count;    // blocks of a posting kernel that are done; 0 between launches
   int last_iters_nbc = 0, last_iters_dbc = 0;
   int64_t n_rhs = 0;
   int64_t launches = 0;         // kernels launched by this handle
@@ -332,6 +375,16 @@ struct nmg_handle {
   if (prof_slot__ >= 0) (h)->prof.end((h)->stream, prof_slot__)
 
 namespace nmg {
+// After all of the grid's writes to HostPost::res() by this block, or in the
+// block that saw the others done: the host may read them.
+__device__ __forceinline__ void post_flag(unsigned long long *flag, unsigned long long seq) {
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    *(volatile unsigned long long *)flag = seq;
+  }
+}
 // Sum over the L neighbouring lanes that share a matrix row (each gets it).
 template <int L>
 __device__ __forceinline__ double lane_sum(double v) {
@@ -400,6 +453,7 @@ int jac_demag_solve(nmg_handle *P, JacDemag &J, double rtol);
 // to max(rtol |b|, atol).
 int nd_prepare(nmg_handle *h);
 bool nd_available(const nmg_handle *h, int mode);
+int post_fields(nmg_handle *h, double *fields, double *scalars);
 int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32,
              const NdOut &out = NdOut());
 void nd_reset_barrier(nmg_handle *h);   // after a launch whose barrier gave up

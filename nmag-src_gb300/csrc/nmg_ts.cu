@@ -205,16 +205,6 @@ __device__ __forceinline__ bool red_grid(const double (&v)[K], int nv, const Red
   if (threadIdx.x == 0) *r.count = 0;
   return true;
 }
-// After the writes to r.host by any threads of the block: the host may read them.
-__device__ __forceinline__ void red_post(const Red &r) {
-  __threadfence_system();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence_system();
-    *(volatile unsigned long long *)r.flag = r.seq;
-  }
-}
-
 // mode 0: sum (x w)^2 ; mode 1: sum x y ; mode 2: max x -> r.host[0]
 template <int kMode>
 __global__ void __launch_bounds__(256) k_red(int n, const double *__restrict__ x, const double *__restrict__ y, Red r) {
@@ -233,7 +223,7 @@ __global__ void __launch_bounds__(256) k_red(int n, const double *__restrict__ x
     step(x0, y0); step(x1, y1); step(x2, y2); step(x3, y3);
   }
   for (; i < n; i += stride) step(x[i], y[i]);
-  if (red_grid<1, kMode == 2>(acc, 1, r, [&](int, double s) { r.host[0] = s; })) red_post(r);
+  if (red_grid<1, kMode == 2>(acc, 1, r, [&](int, double s) { r.host[0] = s; })) post_flag(r.flag, r.seq);
 }
 
 struct VecPtrs { const double *v[kRedMax]; };
@@ -303,7 +293,7 @@ __global__ void __launch_bounds__(256) k_orth_norm(int n, int nv, VecPtrs V, con
   }
   if (red_grid<1>(acc, 1, r, [&](int, double s) { r.host[nh] = s; })) {
     for (int k = threadIdx.x; k < nh; k += blockDim.x) r.host[k] = hcol[k];
-    red_post(r);
+    post_flag(r.flag, r.seq);
   }
 }
 // x += sum_k c_k V_k with the coefficients passed by value (no host-to-device
@@ -352,7 +342,7 @@ __global__ void __launch_bounds__(256)
       acc[1] += q * q;
     }
   }
-  if (red_grid<2>(acc, 2, r, [&](int k, double s) { r.host[k] = s; })) red_post(r);
+  if (red_grid<2>(acc, 2, r, [&](int k, double s) { r.host[k] = s; })) post_flag(r.flag, r.seq);
 }
 // End of one: the correction b = (x0 + sum_k c_k V_k) / ewt (x0 null: 0) or, kRes,
 // b = x0 as it is; acor += b, y = zn0 + acor, and the sum (b ewt)^2 for the host.
@@ -372,7 +362,7 @@ __global__ void __launch_bounds__(256)
     acor[i] = a;
     y[i] = zn0[i] + a;
   }
-  if (red_grid<1>(acc, 1, r, [&](int, double t) { r.host[0] = t; })) red_post(r);
+  if (red_grid<1>(acc, 1, r, [&](int, double t) { r.host[0] = t; })) post_flag(r.flag, r.seq);
 }
 // F.template operator()<NVM>() for the smallest NVM >= nv
 template <class F>
@@ -684,8 +674,7 @@ struct Integrator {
   double *zn[QMAXB + 2];
   std::vector<double *> V;
   DevBuf<unsigned> redcnt;
-  double *hpin = nullptr;  // pinned results of the reductions, after the sequence number's line
-  unsigned long long seq = 0;
+  HostPost post;
   double eta_due = 1.0;    // the next prediction rescales the history by this
   bool ewt_due = false;    // and forms the error weights first
   // CVODE state
@@ -702,22 +691,12 @@ struct Integrator {
   cudaStream_t s() const { return hd->stream; }
   ZnPtrs znp() const { ZnPtrs z; for (int j = 0; j < QMAXB + 2; ++j) z.z[j] = zn[j]; return z; }
 
-  double *res() const { return hpin + 8; }
+  double *res() const { return post.res(); }
   Red red(bool host = true) {
-    if (host) ++seq;
-    return Red{part.p, redcnt.p, res(), reinterpret_cast<unsigned long long *>(hpin), seq};
+    if (host) ++post.seq;
+    return Red{part.p, redcnt.p, res(), post.flag(), post.seq};
   }
-  // Waits for the last reduction's results; false if its kernel did not run.
-  bool wait() {
-    for (unsigned spins = 1;; ++spins) {
-      if (__atomic_load_n(reinterpret_cast<unsigned long long *>(hpin), __ATOMIC_ACQUIRE) == seq) return true;
-      if (spins & 0xfff) continue;
-      const cudaError_t e = cudaStreamQuery(s());   // a launch that failed never posts
-      if (e != cudaErrorNotReady)
-        return e == cudaSuccess &&
-               __atomic_load_n(reinterpret_cast<unsigned long long *>(hpin), __ATOMIC_ACQUIRE) == seq;
-    }
-  }
+  bool wait() { return post.wait(s()); }
   double wrms(const double *x, const double *w) {
     k_red<0><<<red_blocks(n), 256, 0, s()>>>(n, x, w, red()); ++hd->launches;
     if (!wait()) { status = 100; return 0.0; }
@@ -1335,8 +1314,7 @@ Integrator *ts_create(nmg_handle *h, int qmax, int maxl, double rtol, double ato
   ok = ok && I->redcnt.alloc(1) == cudaSuccess && cudaMemset(I->redcnt.p, 0, sizeof(unsigned)) == cudaSuccess;
   ok = ok && I->hdev.alloc(I->maxl + 64) == cudaSuccess;
   ok = ok && I->hcol.alloc(I->maxl + 64) == cudaSuccess;
-  ok = ok && cudaMallocHost(&I->hpin, sizeof(double) * (I->maxl + 64)) == cudaSuccess;
-  if (ok) std::memset(I->hpin, 0, sizeof(double) * (I->maxl + 64));
+  ok = ok && I->post.reserve(I->maxl + 8);
   if (!ok) { ts_destroy(I); return nullptr; }
   for (int j = 0; j < QMAXB + 2; ++j) I->zn[j] = j <= I->qmax + 1 ? I->znbuf.p + n * j : nullptr;
   I->V.resize(I->maxl + 1);
@@ -1356,7 +1334,6 @@ void ts_set_tolerances(Integrator *I, double rtol, double atol) { I->rtol = rtol
 
 void ts_destroy(Integrator *I) {
   if (!I) return;
-  if (I->hpin) cudaFreeHost(I->hpin);
   delete I;
 }
 

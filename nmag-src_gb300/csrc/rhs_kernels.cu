@@ -2313,8 +2313,22 @@ __global__ void k_energy(int N, const double *__restrict__ m, const double *__re
 }
 
 // Block partial sums of V_i, V_i m_i (3) and V_i E_k,i (5): 9 columns.
-__global__ void k_avg_partials(int N, const double *__restrict__ m, const double *__restrict__ vol,
-                               const double *__restrict__ E, double *__restrict__ part, size_t estride) {
+// The block that finishes last goes on to add the blocks' partials.
+__device__ __forceinline__ bool last_block(unsigned *count) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+    if (last) *count = 0;
+  }
+  __syncthreads();
+  __threadfence();
+  return last;
+}
+__global__ void k_avg(int N, const double *__restrict__ m, const double *__restrict__ vol,
+                      const double *__restrict__ E, double *part, size_t estride, unsigned *count, double *host,
+                      unsigned long long *flag, unsigned long long seq) {
   __shared__ double smem[32 * 9];
   double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
@@ -2325,10 +2339,18 @@ __global__ void k_avg_partials(int N, const double *__restrict__ m, const double
   }
   block_sum<9>(v, smem);
   if (threadIdx.x == 0) for (int j = 0; j < 9; ++j) part[9 * blockIdx.x + j] = v[j];
+  if (!last_block(count)) return;
+  if (threadIdx.x < 9) {
+    double t = 0.0;
+#pragma unroll 8
+    for (int b = 0; b < (int)gridDim.x; ++b) t += __ldcg(part + 9 * b + threadIdx.x);
+    host[threadIdx.x] = t;
+  }
+  post_flag(flag, seq);
 }
 
-__global__ void k_maxdm_partials(int N, const double *__restrict__ a, const double *__restrict__ b,
-                                 double *__restrict__ part) {
+__global__ void k_maxdm(int N, const double *__restrict__ a, const double *__restrict__ b, double *part,
+                        unsigned *count, double *host, unsigned long long *flag, unsigned long long seq) {
   __shared__ double smem[32];
   double mx = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
@@ -2344,6 +2366,34 @@ __global__ void k_maxdm_partials(int N, const double *__restrict__ a, const doub
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, smem[w]);
     part[blockIdx.x] = r;
   }
+  if (!last_block(count)) return;
+  if (threadIdx.x == 0) {
+    double r = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < (int)gridDim.x; ++k) r = fmax(r, __ldcg(part + k));
+    host[0] = r;
+  }
+  post_flag(flag, seq);
+}
+// The fields of an evaluation, its error words and iteration counts to the host:
+// values 0..2, then from 8 on the arrays that are asked for, one after another.
+struct PostFields { const double *src[7]; long long n[7]; const int *err, *err2, *iters; };
+__global__ void __launch_bounds__(256) k_post_fields(PostFields a, unsigned *count, double *__restrict__ host,
+                                                     unsigned long long *flag, unsigned long long seq) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  double *o = host + 8;
+#pragma unroll
+  for (int k = 0; k < 7; ++k) {
+    for (long long i = t; i < a.n[k]; i += nt) o[i] = a.src[k][i];
+    o += a.n[k];
+  }
+  if (t == 0) {
+    host[0] = (double)(*a.err | (a.err2 ? *a.err2 : 0));
+    host[1] = (double)a.iters[0];
+    host[2] = (double)a.iters[1];
+  }
+  __threadfence_system();
+  if (last_block(count)) post_flag(flag, seq);
 }
 
 // Solver ordering and two-level data, built once on the host:
@@ -3328,21 +3378,66 @@ int energy_density(nmg_handle *h, const double *d_m, double *d_E5) {
   return cudaGetLastError() == cudaSuccess ? 0 : 100;
 }
 
+// Room for a post of n values; false: no memory.
+static bool post_ready(nmg_handle *h, size_t n) {
+  if (!h->post_count.p) {
+    if (h->post_count.alloc(1) != cudaSuccess ||
+        cudaMemsetAsync(h->post_count.p, 0, sizeof(unsigned), h->stream) != cudaSuccess) {
+      h->post_count.release();
+      return false;
+    }
+  }
+  return h->post.reserve(n);
+}
+
+// The fields (5 x 3 per node), phi and rho of the evaluation just launched, its
+// errors and iteration counts.  Up to kPostMax values in one kernel through
+// pinned memory; -1: too many, the caller copies.
+// Nine synchronised readbacks took 110 us of a cube's 258 us evaluation (now 120 in
+// all), and the film's copies into fresh arrays 0.4 ms more than a kernel and a memcpy.
+constexpr size_t kPostMax = 1 << 20;
+int post_fields(nmg_handle *h, double *fields, double *scalars) {
+  Workspace &W = h->ws;
+  const size_t N = (size_t)h->mesh.N * h->nrep, nf = fields ? 3 * N : 0, ns = scalars ? N : 0, n = 5 * nf + 2 * ns;
+  if (n > kPostMax || !post_ready(h, n + 8)) return -1;
+  PostFields a;
+  const double *src[7] = {W.h_exch, W.h_demag, W.h_anis, W.h_total, W.dmdt, W.phi, W.rho};
+  for (int k = 0; k < 7; ++k) {
+    a.src[k] = src[k];
+    a.n[k] = (long long)(k < 5 ? nf : ns);
+  }
+  a.err = W.err; a.err2 = h->pot ? h->pot->ws.err.p : nullptr; a.iters = W.iters;
+  const int blocks = (int)std::min<size_t>(2 * (size_t)h->sm_count, std::max<size_t>(1, (n + 255) / 256));
+  k_post_fields<<<blocks, 256, 0, h->stream>>>(a, h->post_count, h->post.res(), h->post.flag(), ++h->post.seq);
+  ++h->launches;
+  const bool came = h->post.wait(h->stream);
+  const double *r = h->post.res();
+  if (!came || r[0] != 0.0) {
+    const int rc = check_device_error(h, "nmg_eval_fields");
+    if (rc) return rc;
+    if (!came) {
+      h->last_error = "nmg_eval_fields: launch failed";
+      return 100;
+    }
+  }
+  if (fields) std::memcpy(fields, r + 8, sizeof(double) * 5 * nf);
+  if (scalars) std::memcpy(scalars, r + 8 + 5 * nf, sizeof(double) * 2 * ns);
+  h->last_iters_nbc = (int)r[1];
+  h->last_iters_dbc = (int)r[2];
+  return 0;
+}
+
 int averages(nmg_handle *h, const double *d_m, double avg[3], double energies[5], int member) {
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   const int nblocks = 64;
   const double *E = energies ? W.E5.p + (size_t)member * M.N : nullptr;
+  if (!post_ready(h, 16)) return 100;
   if (energies && energy_density(h, d_m, W.E5)) return 100;
-  k_avg_partials<<<nblocks, 256, 0, h->stream>>>(M.N, d_m + (size_t)member * 3 * M.N, M.vol, E, W.red,
-                                                 (size_t)M.N * h->nrep); ++h->launches;
-  std::vector<double> part(9 * nblocks);
-  if (cudaMemcpyAsync(part.data(), W.red.p, sizeof(double) * 9 * nblocks, cudaMemcpyDeviceToHost, h->stream) ||
-      cudaStreamSynchronize(h->stream))
-    return 100;
-  double tot[9] = {0};
-  for (int b = 0; b < nblocks; ++b)
-    for (int j = 0; j < 9; ++j) tot[j] += part[9 * b + j];
+  k_avg<<<nblocks, 256, 0, h->stream>>>(M.N, d_m + (size_t)member * 3 * M.N, M.vol, E, W.red, (size_t)M.N * h->nrep,
+                                        h->post_count, h->post.res(), h->post.flag(), ++h->post.seq); ++h->launches;
+  if (!h->post.wait(h->stream)) return 100;
+  const double *tot = h->post.res();
   for (int d = 0; d < 3; ++d) avg[d] = tot[1 + d] / tot[0];
   if (energies) for (int k = 0; k < 5; ++k) energies[k] = tot[4 + k];
   return 0;
@@ -3350,14 +3445,11 @@ int averages(nmg_handle *h, const double *d_m, double avg[3], double energies[5]
 
 int max_dm(nmg_handle *h, const double *d_m, const double *d_mprev, double *out) {
   const int nblocks = 64;
-  k_maxdm_partials<<<nblocks, 256, 0, h->stream>>>(h->mesh.N * h->nrep, d_m, d_mprev, h->ws.red); ++h->launches;
-  double part[nblocks];
-  if (cudaMemcpyAsync(part, h->ws.red.p, sizeof(double) * nblocks, cudaMemcpyDeviceToHost, h->stream) ||
-      cudaStreamSynchronize(h->stream))
-    return 100;
-  double mx = 0.0;
-  for (int b = 0; b < nblocks; ++b) mx = part[b] > mx ? part[b] : mx;
-  *out = mx;
+  if (!post_ready(h, 16)) return 100;
+  k_maxdm<<<nblocks, 256, 0, h->stream>>>(h->mesh.N * h->nrep, d_m, d_mprev, h->ws.red, h->post_count, h->post.res(),
+                                          h->post.flag(), ++h->post.seq); ++h->launches;
+  if (!h->post.wait(h->stream)) return 100;
+  *out = h->post.res()[0];
   return 0;
 }
 
