@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kT) k_llg_vjp(VjpArgs a) {
     __syncthreads();
     if (threadIdx.x < 3) {
       double s = 0.0;
-      for (int q = 0; q < kT / 32; ++q) s += sm[threadIdx.x][q];
+      for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += sm[threadIdx.x][q];
       a.hsum[3 * blockIdx.x + threadIdx.x] = s;
     }
   }
@@ -248,18 +248,19 @@ __global__ void k_pulse_acc(int nparts, const double *__restrict__ hsum, double 
 }
 
 // ub += -c_exch Kx (Hb / V) (Kx symmetric); phibar = -sum_c G_c^T (Hb_c / V).
+template <int L>
 __global__ void k_adj_spmv(int N, int nnz, const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col_idx,
                            const int32_t *__restrict__ tpos, const double *__restrict__ Kx,
-                           const double *__restrict__ G, const double *__restrict__ vol,
+                           const double *__restrict__ G, const double *__restrict__ ivol,
                            const double *__restrict__ Hb, double c_exch, int do_demag, double *__restrict__ ub,
                            double *__restrict__ phibar) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L;
   if (i >= N) return;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, p = 0.0;
-  for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k) {
+  for (int k = row_ptr[i] + threadIdx.x % L, end = row_ptr[i + 1]; k < end; k += L) {
     const int j = col_idx[k];
     const double *hj = Hb + 3 * (size_t)j;
-    const double iv = 1.0 / vol[j];
+    const double iv = ivol[j];
     const double h0 = hj[0] * iv, h1 = hj[1] * iv, h2 = hj[2] * iv;
     const double kv = Kx[k];
     s0 += kv * h0; s1 += kv * h1; s2 += kv * h2;
@@ -268,6 +269,9 @@ __global__ void k_adj_spmv(int N, int nnz, const int32_t *__restrict__ row_ptr, 
       p += (G[tk] * h0 + G[(size_t)nnz + tk] * h1) + G[2 * (size_t)nnz + tk] * h2;
     }
   }
+  s0 = lane_sum<L>(s0); s1 = lane_sum<L>(s1); s2 = lane_sum<L>(s2);
+  if (do_demag) p = lane_sum<L>(p);
+  if (threadIdx.x % L) return;
   ub[3 * (size_t)i] -= c_exch * s0;
   ub[3 * (size_t)i + 1] -= c_exch * s1;
   ub[3 * (size_t)i + 2] -= c_exch * s2;
@@ -286,19 +290,21 @@ __global__ void k_adj_dbc(int N, const int32_t *__restrict__ b_of_node, const do
 }
 
 // phibar2b_j = phibar_n - (K_BI z_I)_n, n = node_of_b[j]
+template <int L>
 __global__ void k_adj_bnd(int nb, const int32_t *__restrict__ node_of_b, const int32_t *__restrict__ b_of_node,
                           const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col_idx,
                           const double *__restrict__ K, const double *__restrict__ z,
                           const double *__restrict__ phibar, double *__restrict__ out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) / L;
   if (j >= nb) return;
   const int n = node_of_b[j];
   double s = 0.0;
-  for (int k = row_ptr[n]; k < row_ptr[n + 1]; ++k) {
+  for (int k = row_ptr[n] + threadIdx.x % L, end = row_ptr[n + 1]; k < end; k += L) {
     const int c = col_idx[k];
     if (b_of_node[c] < 0) s += K[k] * z[c];
   }
-  out[j] = phibar[n] - s;
+  s = lane_sum<L>(s);
+  if (threadIdx.x % L == 0) out[j] = phibar[n] - s;
 }
 
 // B^T y over the row-major BEM: warp (group g, slab s) owns 128 columns
@@ -387,12 +393,26 @@ __global__ void __launch_bounds__(kT) k_gemv_t_df(int nb, int ld, int groups, in
   for (int c = 0; c < 8; ++c) out[c] = (double)S[c] + (double)C[c];
 }
 
-__global__ void k_col_sum(int nb, int ld, int slabs, const double *__restrict__ part, double *__restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nb) return;
+// out_c = sum of the slabs' partials: 32 columns by 8 parts of the slabs a block
+// (a thread per column added them one after another: 79 us for 602 columns and
+// slabs, 4.4 now with 75).
+__global__ void __launch_bounds__(256) k_col_sum(int nb, int ld, int slabs, const double *__restrict__ part,
+                                                 double *__restrict__ out) {
+  __shared__ double sm[8][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (int sl = 0; sl < slabs; ++sl) s += part[(size_t)sl * ld + c];
-  out[c] = s;
+  if (c < nb) {
+#pragma unroll 8
+    for (int sl = g; sl < slabs; sl += 8) s += part[(size_t)sl * ld + c];
+  }
+  sm[g][lane] = s;
+  __syncthreads();
+  if (g == 0 && c < nb) {
+    double t = sm[0][lane];
+#pragma unroll
+    for (int q = 1; q < 8; ++q) t += sm[q][lane];
+    out[c] = t;
+  }
 }
 
 // Neumann adjoint right-hand side: phibar + scatter(B^T phibar2b)
@@ -405,17 +425,20 @@ __global__ void k_adj_scatter(int N, const int32_t *__restrict__ b_of_node, cons
 }
 
 // ub_j += -Ms sum_i Dx_d[i][j] rhobar_i
+template <int L>
 __global__ void k_adj_div(int N, int nnz, double Ms, const int32_t *__restrict__ row_ptr,
                           const int32_t *__restrict__ col_idx, const int32_t *__restrict__ tpos,
                           const double *__restrict__ Dx, const double *__restrict__ rhobar, double *__restrict__ ub) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / L;
   if (i >= N) return;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-  for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k) {
+  for (int k = row_ptr[i] + threadIdx.x % L, end = row_ptr[i + 1]; k < end; k += L) {
     const int tk = tpos[k];
     const double r = rhobar[col_idx[k]];
     s0 += Dx[tk] * r; s1 += Dx[(size_t)nnz + tk] * r; s2 += Dx[2 * (size_t)nnz + tk] * r;
   }
+  s0 = lane_sum<L>(s0); s1 = lane_sum<L>(s1); s2 = lane_sum<L>(s2);
+  if (threadIdx.x % L) return;
   ub[3 * (size_t)i] -= Ms * s0;
   ub[3 * (size_t)i + 1] -= Ms * s1;
   ub[3 * (size_t)i + 2] -= Ms * s2;
@@ -423,7 +446,7 @@ __global__ void k_adj_div(int N, int nnz, double Ms, const int32_t *__restrict__
 
 // Per-element parameter cotangents of one stage (one thread per tet, no atomics).
 __global__ void k_elem_grad(int T, const int32_t *__restrict__ tets, const double *__restrict__ dL,
-                            const double *__restrict__ adet, const double *__restrict__ vol,
+                            const double *__restrict__ adet, const double *__restrict__ ivol,
                             const double *__restrict__ u, const double *__restrict__ Hb,
                             const double *__restrict__ rhobar, const double *__restrict__ sanis, double c_exch,
                             double Ms, double *__restrict__ gwK, double *__restrict__ gwD,
@@ -437,7 +460,7 @@ __global__ void k_elem_grad(int T, const int32_t *__restrict__ tets, const doubl
     double acc = 0.0;
     for (int a = 0; a < 4; ++a) {
       const double *ha = Hb + 3 * (size_t)v[a];
-      const double iva = 1.0 / vol[v[a]];
+      const double iva = ivol[v[a]];
       for (int b = 0; b < 4; ++b) {
         const double *ubv = u + 3 * (size_t)v[b];
         const double kab = kc * ((g[3 * a] * g[3 * b] + g[3 * a + 1] * g[3 * b + 1]) + g[3 * a + 2] * g[3 * b + 2]);
@@ -457,7 +480,7 @@ __global__ void k_elem_grad(int T, const int32_t *__restrict__ tets, const doubl
   }
   if (gkap && sanis) {
     double acc = 0.0;
-    for (int a = 0; a < 4; ++a) acc += sanis[v[a]] / vol[v[a]];
+    for (int a = 0; a < 4; ++a) acc += sanis[v[a]] * ivol[v[a]];
     gkap[t] += gc * acc;
   }
 }
@@ -544,7 +567,8 @@ int stage_vjp(nmg_handle *h, Tape &T, const double *u, const double *H, const do
   cudaStream_t s = h->stream;
   const int N = M.N;
   const int demag = (h->opt.do_demag && M.nb > 0) ? 1 : 0;
-  const int nparts = nblk(N, kT);
+  // small meshes over more SMs (FP64-bound); larger ones with fewer partial sums
+  const int vt = N <= kRowLanesMax ? 64 : kT, nparts = nblk(N, vt);
   VjpArgs a;
   a.N = N;
   a.anis_on = (h->ep.active || mt.K1 != 0.0) ? 1 : 0;
@@ -554,20 +578,20 @@ int stage_vjp(nmg_handle *h, Tape &T, const double *u, const double *H, const do
   a.ay = h->ep.active ? h->ep.axis[1] : mt.axis[1];
   a.az = h->ep.active ? h->ep.axis[2] : mt.axis[2];
   a.ub = ub; a.Hb = T.Hbar; a.sanis = T.sanis; a.hsum = G.gpul ? T.hsum.p : nullptr;
-  k_llg_vjp<<<nparts, kT, 0, s>>>(a);
+  k_llg_vjp<<<nparts, vt, 0, s>>>(a);
   ADJ_TRY(launched(h, "llg vjp"));
   if (G.gpul && T.npulses > 0 && T.spp > 0 && step / T.spp < T.npulses) {
     k_pulse_acc<<<1, 32, 0, s>>>(nparts, T.hsum, G.gpul + 3 * (size_t)(step / T.spp));
     ADJ_TRY(launched(h, "pulse cotangent"));
   }
-  k_adj_spmv<<<nblk(N, kT), kT, 0, s>>>(N, M.nnz, M.row_ptr, M.col_idx, h->ep.tpos, h->exch_K(), M.G, M.vol, T.Hbar,
+  NMG_LAUNCH_ROWS(k_adj_spmv, N, N, s, N, M.nnz, M.row_ptr, M.col_idx, h->ep.tpos, h->exch_K(), M.G, M.ivol, T.Hbar,
                                         mt.exch_coeff, demag, ub, T.phibar);
   ADJ_TRY(launched(h, "exchange/grad adjoint"));
   if (demag) {
     k_adj_dbc<<<nblk(N, kT), kT, 0, s>>>(N, M.b_of_node, T.phibar, T.rhs, T.z);
     ADJ_TRY(launched(h, "adjoint dirichlet rhs"));
     if (cg_solve(h, 3, T.rhs, T.z, h->opt.dbc_rtol, h->opt.dbc_atol, h->opt.dbc_maxits)) return 100;
-    k_adj_bnd<<<nblk(M.nb, kT), kT, 0, s>>>(M.nb, M.node_of_b, M.b_of_node, M.row_ptr, M.col_idx, M.K, T.z, T.phibar,
+    NMG_LAUNCH_ROWS(k_adj_bnd, N, M.nb, s, M.nb, M.node_of_b, M.b_of_node, M.row_ptr, M.col_idx, M.K, T.z, T.phibar,
                                            T.y2b);
     ADJ_TRY(launched(h, "adjoint boundary"));
     const bool df = h->opt.bem_precision == 2 && M.bem16lo.p && T.yhl.p;
@@ -582,17 +606,19 @@ int stage_vjp(nmg_handle *h, Tape &T, const double *u, const double *H, const do
                                                                                     T.t_rows, M.bem, T.y2b, T.tpart);
     }
     ADJ_TRY(launched(h, "BEM transpose product"));
-    k_col_sum<<<nblk(M.nb, kT), kT, 0, s>>>(M.nb, M.ld, df ? T.d_slabs : T.t_slabs, T.tpart, T.y1b);
+    k_col_sum<<<nblk(M.nb, 32), 256, 0, s>>>(M.nb, M.ld, df ? T.d_slabs : T.t_slabs, T.tpart, T.y1b);
     ADJ_TRY(launched(h, "BEM transpose sum"));
     k_adj_scatter<<<nblk(N, kT), kT, 0, s>>>(N, M.b_of_node, T.phibar, T.y1b, T.rhs);
     ADJ_TRY(launched(h, "adjoint neumann rhs"));
     if (cg_solve(h, 2, T.rhs, T.rhobar, h->opt.nbc_rtol, h->opt.nbc_atol, h->opt.nbc_maxits)) return 100;
-    k_adj_div<<<nblk(N, kT), kT, 0, s>>>(N, M.nnz, mt.Ms, M.row_ptr, M.col_idx, h->ep.tpos,
+    NMG_LAUNCH_ROWS(k_adj_div, N, N, s, N, M.nnz, mt.Ms, M.row_ptr, M.col_idx, h->ep.tpos,
                                          h->ep.active ? h->ep.Dx.p : M.D.p, T.rhobar, ub);
     ADJ_TRY(launched(h, "div adjoint"));
   }
   if (G.gwK || G.gwD || G.gkap) {
-    k_elem_grad<<<nblk(M.T, kT), kT, 0, s>>>(M.T, M.tets, M.dL, M.adet, M.vol, u, T.Hbar,
+    // one-warp blocks: FP64-bound, and the cube's 6,000 elements in blocks of 256
+    // sat on 24 SMs (27 us; 13 so, the volumes' reciprocals being read)
+    k_elem_grad<<<nblk(M.T, 32), 32, 0, s>>>(M.T, M.tets, M.dL, M.adet, M.ivol, u, T.Hbar,
                                              demag ? T.rhobar.p : nullptr, T.sanis, mt.exch_coeff, mt.Ms, G.gwK,
                                              G.gwD, G.gkap);
     ADJ_TRY(launched(h, "element cotangents"));
@@ -696,7 +722,7 @@ int rk4_forward(nmg_handle *h, const double *d_m0, double dt, int nsteps, int ck
     if (M.ld > 0) {
       T.t_groups = (M.ld / 4 + 31) / 32;
       const int target = 64 * h->sm_count;
-      int slabs = std::max(1, std::min(M.nb, target / std::max(1, T.t_groups)));
+      int slabs = std::max(1, std::min(M.nb / 8, target / std::max(1, T.t_groups)));   // 8 rows or more each
       T.t_rows = (M.nb + slabs - 1) / slabs;
       T.t_slabs = (M.nb + T.t_rows - 1) / T.t_rows;
       size_t part_slabs = T.t_slabs;
@@ -763,7 +789,7 @@ int rk4_adjoint(nmg_handle *h, const double *d_mT_bar, const double *d_hist_bar,
   if (!T.su.p) {
     if (T.su.alloc((size_t)T.ckpt * 4 * n3) || T.sH.alloc((size_t)T.ckpt * 4 * n3) || T.lam.alloc(n3) ||
         T.kb.alloc(n3) || T.ub.alloc(n3) || T.acc.alloc(n3) || T.Hbar.alloc(n3) || T.sanis.alloc(N) ||
-        T.hsum.alloc(3 * (size_t)nblk(N, kT)) || T.phibar.alloc(N) || T.rhs.alloc(N) || T.z.alloc(N) ||
+        T.hsum.alloc(3 * (size_t)nblk(N, 64)) || T.phibar.alloc(N) || T.rhs.alloc(N) || T.z.alloc(N) ||
         T.rhobar.alloc(N) || T.y2b.alloc(std::max(M.nb, 1)) || T.y1b.alloc(std::max(M.nb, 1))) {
       h->last_error = "rk4 adjoint: device allocation failed";
       return 100;
