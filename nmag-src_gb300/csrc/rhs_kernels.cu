@@ -2326,6 +2326,7 @@ __device__ __forceinline__ bool last_block(unsigned *count) {
   __threadfence();
   return last;
 }
+constexpr int kAvgBlocks = 64;   // two partials a lane in the last block
 __global__ void k_avg(int N, const double *__restrict__ m, const double *__restrict__ vol,
                       const double *__restrict__ E, double *part, size_t estride, unsigned *count, double *host,
                       unsigned long long *flag, unsigned long long seq) {
@@ -2340,11 +2341,18 @@ __global__ void k_avg(int N, const double *__restrict__ m, const double *__restr
   block_sum<9>(v, smem);
   if (threadIdx.x == 0) for (int j = 0; j < 9; ++j) part[9 * blockIdx.x + j] = v[j];
   if (!last_block(count)) return;
-  if (threadIdx.x < 9) {
-    double t = 0.0;
-#pragma unroll 8
-    for (int b = 0; b < (int)gridDim.x; ++b) t += __ldcg(part + 9 * b + threadIdx.x);
-    host[threadIdx.x] = t;
+  if (threadIdx.x < 32) {   // nine trees over the 64 blocks (chains of 64 FP64 adds: 6,000 clocks)
+    double t[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j)
+      t[j] = __ldcg(part + 9 * threadIdx.x + j) + __ldcg(part + 9 * (threadIdx.x + 32) + j);
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+#pragma unroll
+      for (int j = 0; j < 9; ++j) t[j] += __shfl_xor_sync(0xffffffffu, t[j], o);
+#pragma unroll
+    for (int j = 0; j < 9; ++j)
+      if ((int)threadIdx.x == j) host[j] = t[j];
   }
   post_flag(flag, seq);
 }
@@ -2367,11 +2375,10 @@ __global__ void k_maxdm(int N, const double *__restrict__ a, const double *__res
     part[blockIdx.x] = r;
   }
   if (!last_block(count)) return;
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-#pragma unroll 8
-    for (int k = 0; k < (int)gridDim.x; ++k) r = fmax(r, __ldcg(part + k));
-    host[0] = r;
+  if (threadIdx.x < 32) {
+    double r = fmax(__ldcg(part + threadIdx.x), __ldcg(part + threadIdx.x + 32));
+    for (int o = 16; o; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+    if (threadIdx.x == 0) host[0] = r;
   }
   post_flag(flag, seq);
 }
@@ -3372,7 +3379,7 @@ int energy_density(nmg_handle *h, const double *d_m, double *d_E5) {
   Workspace &W = h->ws;
   const nmg_material &mt = h->mat;
   const int NB = M.N * h->nrep;   // pointwise over all members: E[k * NB + member * N + i]
-  k_energy<<<nblk(NB, 256), 256, 0, h->stream>>>(NB, d_m, W.h_exch, W.h_demag, W.h_ext, mt.E_coeff_half,
+  k_energy<<<nblk(NB, 64), 64, 0, h->stream>>>(NB, d_m, W.h_exch, W.h_demag, W.h_ext, mt.E_coeff_half,
                                                   mt.E_coeff_ext, mt.K1, mt.axis[0], mt.axis[1], mt.axis[2],
                                                   h->ap.ne, h->ap.epow, h->ap.ecoef, d_E5); ++h->launches;
   return cudaGetLastError() == cudaSuccess ? 0 : 100;
@@ -3430,11 +3437,11 @@ int post_fields(nmg_handle *h, double *fields, double *scalars) {
 int averages(nmg_handle *h, const double *d_m, double avg[3], double energies[5], int member) {
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
-  const int nblocks = 64;
+  const int nblocks = kAvgBlocks, threads = M.N <= 64 * nblocks ? 64 : 256;   // (two warps share an FP64 pipe better)
   const double *E = energies ? W.E5.p + (size_t)member * M.N : nullptr;
   if (!post_ready(h, 16)) return 100;
   if (energies && energy_density(h, d_m, W.E5)) return 100;
-  k_avg<<<nblocks, 256, 0, h->stream>>>(M.N, d_m + (size_t)member * 3 * M.N, M.vol, E, W.red, (size_t)M.N * h->nrep,
+  k_avg<<<nblocks, threads, 0, h->stream>>>(M.N, d_m + (size_t)member * 3 * M.N, M.vol, E, W.red, (size_t)M.N * h->nrep,
                                         h->post_count, h->post.res(), h->post.flag(), ++h->post.seq); ++h->launches;
   if (!h->post.wait(h->stream)) return 100;
   const double *tot = h->post.res();
@@ -3444,7 +3451,7 @@ int averages(nmg_handle *h, const double *d_m, double avg[3], double energies[5]
 }
 
 int max_dm(nmg_handle *h, const double *d_m, const double *d_mprev, double *out) {
-  const int nblocks = 64;
+  const int nblocks = kAvgBlocks;
   if (!post_ready(h, 16)) return 100;
   k_maxdm<<<nblocks, 256, 0, h->stream>>>(h->mesh.N * h->nrep, d_m, d_mprev, h->ws.red, h->post_count, h->post.res(),
                                           h->post.flag(), ++h->post.seq); ++h->launches;
