@@ -979,10 +979,16 @@ int set_threads(nmg_batch *b, int threads) {
   cudaFuncSetAttribute(nmg::k_batch_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(b));
   b->threads = threads;
   b->n_team = threads == nmg::kTeamThreads ? b->n_large : 0;   // a team reproduces the sums of that CTA
-  // every resident CTA, but no more than have a particle to work on
+  // every resident CTA, but no more than have a particle to work on: a cluster
+  // for each team and CTAs for the rest, in clusters too, so that no particle
+  // waits for a team's (8 particles of 125 to 729 nodes: 6.6 ms a pass when the
+  // teams' CTAs took the rest on afterwards, 4.2 so)
   const int small = b->P - b->n_team;
-  b->blocks = std::min(std::max(small, nmg::kTeam * b->n_team), per * b->sm_count);
-  if (b->n_team > 0) b->blocks = std::max(1, b->blocks / nmg::kTeam) * nmg::kTeam;
+  b->blocks = std::min(small + nmg::kTeam * b->n_team, per * b->sm_count);
+  if (b->n_team > 0) {
+    b->blocks = std::min((b->blocks + nmg::kTeam - 1) / nmg::kTeam, per * b->sm_count / nmg::kTeam) * nmg::kTeam;
+    b->blocks = std::max(b->blocks, nmg::kTeam);
+  }
   drop_graph(b);
   return 0;
 }
