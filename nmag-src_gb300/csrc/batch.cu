@@ -786,11 +786,15 @@ __device__ int next_particle(const BatchArgs &a, int *sp) {
   __syncthreads();
   return p;
 }
+// The cluster this CTA belongs to, once all of its CTAs have started: a store
+// into the shared memory of one that has not is undefined.
 __device__ Team cluster_team() {
   unsigned rank, size;
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
-  return {(int)rank, (int)size, 0};
+  const Team T = {(int)rank, (int)size, 0};
+  tsync(T);
+  return T;
 }
 
 __global__ void __launch_bounds__(352) k_batch_run(BatchArgs a) {   // 352: the largest CTA a schedule may choose
