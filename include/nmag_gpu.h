@@ -282,8 +282,8 @@ int nmg_rhs_device(nmg_handle *h, const double *d_m, double *d_dmdt);
  * d_x + n * nb) with the handle's BEM in its bem_precision form -- the
  * reference's dense BEM MatMult (nsim.ml:3128-3140) for many right-hand sides
  * at once (with bem_precision 3 one tensor-core product).  On the handle's
- * stream; returns after the product is complete.  Not with the anchored
- * product. */
+ * stream; returns after the product is complete.  d_y may be d_x (in place).
+ * Not with the anchored product. */
 int nmg_bem_apply(nmg_handle *h, const double *d_x, double *d_y, int n_rhs);
 int nmg_rk4_device(nmg_handle *h, double *d_m, double dt, int nsteps);
 

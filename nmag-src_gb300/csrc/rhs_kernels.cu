@@ -1572,10 +1572,10 @@ __global__ void __launch_bounds__(kGemvThreads) k_gemv_f32(int nb, int ld, long 
   }
 }
 
-// y[r] = sum of the partials of the warps whose unit range meets row r, in
 // y = B x for a boundary of fewer rows than k_gemv_f64 has segments, where that
 // splits every row: a block of four warps per row, and no partials to add up in
-// another launch (602 nodes: 11.4 us of two kernels -> 4.4).
+// another launch (602 nodes: 11.4 us of two kernels -> 4.4).  A block writes its
+// row while others still read x, so x and y must not overlap.
 __global__ void __launch_bounds__(128) k_gemv_f64_rows(int nb, int ld, const double *__restrict__ B,
                                                        const double *__restrict__ x, double *__restrict__ y) {
   __shared__ double sm[4];
@@ -1592,6 +1592,8 @@ __global__ void __launch_bounds__(128) k_gemv_f64_rows(int nb, int ld, const dou
   __syncthreads();
   if (threadIdx.x == 0) y[blockIdx.x] = (sm[0] + sm[1]) + (sm[2] + sm[3]);
 }
+
+// y[r] = sum of the partials of the warps whose unit range meets row r, in
 // warp order (Q = units per row).
 __global__ void k_row_sum(int nb, long long Q, long long seg, int maxr, long long nwarps,
                           const double *__restrict__ part, double *__restrict__ y) {
@@ -2901,6 +2903,12 @@ int init_workspace(nmg_handle *h, std::string &err) {
   return 0;
 }
 
+// x[0..n) and y[0..n) have no value in common.
+static bool apart(const double *x, const double *y, size_t n) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y), len = n * sizeof(double);
+  return a + len <= b || b + len <= a;
+}
+
 void bem_gemv(nmg_handle *h, const double *x, double *y) {
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
@@ -2953,7 +2961,7 @@ void bem_gemv(nmg_handle *h, const double *x, double *y) {
     NMG_PROF_BEGIN(h, 0);
     k_gemv_f32<<<W.gemv_blocks, kGemvThreads, 0, h->stream>>>(nb, M.ld, seg, maxr, M.bem32, x32, W.bpart); ++h->launches;
     NMG_PROF_END(h);
-  } else if (nb <= W.gemv_blocks * (kGemvThreads / 32)) {
+  } else if (nb <= W.gemv_blocks * (kGemvThreads / 32) && apart(x, y, nb)) {
     NMG_PROF_BEGIN(h, 0);
     k_gemv_f64_rows<<<nb, 128, 0, h->stream>>>(nb, M.ld, M.bem, x, y); ++h->launches;
     NMG_PROF_END(h);
@@ -3033,10 +3041,12 @@ void bem_apply(nmg_handle *h, const double *x, double *y, int n) {
   const size_t nb = h->mesh.nb;
   size_t off = 0;
   const size_t need = bem_pass_doubles(h, &off);
-  const bool pass = n > 1 && (h->opt.bem_precision == 0 || (h->opt.bem_precision == 2 && h->mesh.bem16lo.p)) &&
+  // A pass reads its vectors before it writes any: in place it answers as one
+  // product after the other, but not where a vector's answer lies on another vector.
+  const bool pass = n > 1 && (x == y || apart(x, y, n * nb)) && (h->opt.bem_precision == 0 || (h->opt.bem_precision == 2 && h->mesh.bem16lo.p)) &&
                     (W.apply_part.n >= need || W.apply_part.alloc(need) == cudaSuccess);
   if (!pass) {
-    cudaGetLastError();   // no room for a pass: vector by vector
+    cudaGetLastError();   // (no room for a pass)
     for (int k = 0; k < n; ++k) bem_gemv(h, x + k * nb, y + k * nb);
     return;
   }
