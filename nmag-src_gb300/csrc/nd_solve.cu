@@ -32,7 +32,15 @@
 //
 // Every solve ends with the FP64 residual b - A x; while it exceeds the
 // tolerance the residual is solved for and added (FP64 factors: none needed
-// down to ~1e-13; FP32 factors: each pass gains 4 to 6 digits).
+// down to ~1e-13; FP32 factors: each pass gains 4 to 6 digits, less on long
+// wires, whose condition number is the square of their length in elements).
+// A residual that no longer falls is the answer's rounding once it is as small
+// as that of |A||x| + |b|, and ends the solve as well (kNdRound): on a wire of
+// L x 1 x 1 cells, magnetised along it, that is 1.5e-12 of |b| for L = 500,
+// 1e-11 for 2,000, 1e-10 for 8,000, and no FP64 answer has a smaller one.  (The
+// FP64 CG's recurrence runs on below it and meets any tolerance; the
+// mixed-precision CG measures its residual and refuses one below rounding, and
+// so do FP32 factors, but for the few units by which two answers' rounding differs.)
 #include <algorithm>
 #include <array>
 #include <cmath>
@@ -50,6 +58,10 @@ constexpr int kNdWorker = 256;
 constexpr int nd_chunk(int mb) { return mb == 8 ? 1024 : 2048; }   // vector entries a worker keeps in shared memory
 constexpr int kNdPanel = 32;                 // pivots eliminated per factorisation step
 constexpr int kNdMaxPass = 11;
+constexpr int kNdProbePass = 8;              // passes the setup's probes may take; more: the CG
+// Residuals that have stopped falling lie at 0.5 to 3 units of rounding
+// (2^-53) of |A||x| + |b|, at 20 on a wire of 16,000 cells.
+constexpr double kNdRound = 64.0 / 9007199254740992.0;
 constexpr int kNdChildren = 8;               // children of a front at most (three merged tree levels)
 constexpr double kLevelSec = 3.5e-6, kEntriesPerSec = 0.3e12;   // the plan's cost model
 constexpr unsigned kNdSpinLimit = 1u << 25;  // seconds; then the error flag ends every block
@@ -394,10 +406,16 @@ __global__ void k_nd_rows(int n, const int32_t *__restrict__ perm, const int32_t
   }
 }
 
-// The setup's right-hand sides: one without structure, or 1 everywhere.
-__global__ void k_nd_probe(int n, double *__restrict__ b, int hash) {
+// The setup's right-hand sides: 1 everywhere, one without structure, one that
+// rises along an axis (the smoothest, whose answer is the largest).
+enum { kProbeOne, kProbeHash, kProbeRise, kProbes };
+__global__ void k_nd_probe(int n, double *__restrict__ b, int kind, const double *__restrict__ X, int axis,
+                           double middle) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = hash ? (double)((unsigned)i * 2654435761u >> 8) / 16777216.0 - 0.5 : 1.0;
+  if (i >= n) return;
+  if (kind == kProbeOne) b[i] = 1.0;
+  else if (kind == kProbeHash) b[i] = (double)((unsigned)i * 2654435761u >> 8) / 16777216.0 - 0.5;
+  else b[i] = X[3 * (size_t)i + axis] - middle;
 }
 
 // one = x (elimination order), kone = K x.
@@ -431,6 +449,7 @@ struct NdArgs {
   unsigned *bar;
   int *err, *iters;
   double rtol, atol;
+  bool probe;                 // whatever the tolerance, down to rounding will do
 };
 
 __device__ __forceinline__ unsigned nd_ld_acquire(const unsigned *p) {
@@ -569,7 +588,8 @@ __global__ void __launch_bounds__(kNdThreads, 1) k_nd_solve(NdArgs a) {
   constexpr int SH = NV == 32 ? 0 : (NV == 16 ? 1 : 2);
   constexpr int MW = MB >= 2 ? 2 : 1, Q = MB / MW; // row work outside the sweeps: Q threads per row, MW members each
   extern __shared__ char nd_dyn[];
-  __shared__ double s_res[2 * MB], s_mean[MB], s_tol[MB], s_floor[MB], s_last[MB];
+  __shared__ double s_res[2 * MB], s_mean[MB], s_tol[MB], s_last[MB];
+  __shared__ double s_size[2 * MB];
   __shared__ int s_state;
   __shared__ double s_sm[kNdThreads / 32 * 2 * MB];
   const int tid = threadIdx.x, half = tid / kNdWorker, wt = tid % kNdWorker;
@@ -761,9 +781,6 @@ __global__ void __launch_bounds__(kNdThreads, 1) k_nd_solve(NdArgs a) {
         const double bn = sqrt(fmax(s_res[MB + tid] - a.N * mean * mean, 0.0));
         s_mean[tid] = mean;
         s_tol[tid] = fmax(a.rtol * bn, a.atol);
-        // FP64 factors: a residual that no longer falls is the answer's rounding
-        // (the CG's own recurrence runs on below it and meets any tolerance)
-        s_floor[tid] = sizeof(T) == 8 ? 1e-10 * bn : -1.0;
         s_last[tid] = 0.0;
       }
       __syncthreads();
@@ -807,18 +824,52 @@ __global__ void __launch_bounds__(kNdThreads, 1) k_nd_solve(NdArgs a) {
     if (!nd_wait(a, epoch)) return;
     nd_total<MB>(slot1, s_res);
     if (tid == 0) {
-      int st = 1;   // 1 done, 0 another pass, 2 failed
+      int st = 1;   // 1 done, 0 another pass, 2 failed, 3 done if what is left is rounding
       for (int m = 0; m < a.nm; ++m) {
         const double rn = sqrt(s_res[m]);
         if (!(rn == rn) || isinf(rn)) st = 2;
-        else if (!(rn <= s_tol[m]) && !(pass > 0 && rn > 0.25 * s_last[m] && rn <= s_floor[m]) && st == 1) st = 0;
+        else if (!(rn <= s_tol[m]) && st != 2)
+          st = st != 0 && pass > 0 && (rn > 0.25 * s_last[m] || pass + 1 >= kNdMaxPass) ? 3 : 0;
         s_last[m] = rn;
       }
-      if (st == 0 && pass + 1 >= kNdMaxPass) st = 2;
       s_state = st;
     }
     __syncthreads();
-    const int st = s_state;
+    int st = s_state;
+    if (st == 3) {   // the same in every block
+#pragma unroll
+      for (int q = 0; q < 2 * MW; ++q) v[q] = 0.0;
+      for (int p = gt / Q; p < a.n; p += gn / Q) {
+        double t[MW], s[MW];
+        const int i = a.perm[a.N + p];
+#pragma unroll
+        for (int w = 0; w < MW; ++w) s[w] = m0 + w < a.nm ? fabs(a.b[(size_t)(m0 + w) * a.N + i]) : 0.0;
+        for (int q = a.prow[p]; q < a.prow[p + 1]; ++q) {
+          ld_members<double, MW>(a.xw + (size_t)a.pcol[q] * MB + m0, t);
+          const double kv = fabs(a.pK[q]);
+#pragma unroll
+          for (int w = 0; w < MW; ++w) s[w] = fma(kv, fabs(t[w]), s[w]);
+        }
+#pragma unroll
+        for (int w = 0; w < MW; ++w) v[w] += s[w] * s[w];
+      }
+      nd_partial<MB, MW>(v, s_sm, slot0);   // (read in the first pass only)
+      nd_arrive(a);
+      if (!nd_wait(a, epoch)) return;
+      nd_total<MB>(slot0, s_size);
+      if (tid == 0) {
+        st = 1;
+        for (int m = 0; m < a.nm; ++m) {
+          double floor = kNdRound * sqrt(s_size[m]);
+          if (sizeof(T) == 4 && !a.probe) floor = fmin(floor, 4.0 * s_tol[m]);
+          if (!(s_last[m] <= fmax(s_tol[m], floor))) st = 0;
+        }
+        s_state = st;
+      }
+      __syncthreads();
+      st = s_state;
+    }
+    if (st == 0 && pass + 1 >= kNdMaxPass) st = 2;
     failed = st == 2;
     if (st != 0) break;
     nd_arrive(a);   // slot1 is free, r is complete
@@ -1197,13 +1248,25 @@ static int nd_setup(nmg_handle *h, std::string &err) {
   cudaGetLastError();
   W.iters.swap(iters);
   W.err.swap(errw);
+  double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
+  for (int i = 0; i < N; ++i)
+    for (int d = 0; d < 3; ++d) {
+      mn[d] = std::min(mn[d], X[3 * (size_t)i + d]);
+      mx[d] = std::max(mx[d], X[3 * (size_t)i + d]);
+    }
+  int axis = 0;
+  for (int d = 1; d < 3; ++d)
+    if (mx[d] - mn[d] > mx[axis] - mn[axis]) axis = d;
+  auto probe = [&](int kind) {
+    k_nd_probe<<<nblk(N, 256), 256, 0, st>>>(N, pb, kind, M.coords, axis, 0.5 * (mn[axis] + mx[axis]));
+  };
   int rc = 0;
   if (D.sys[0].ready) {   // the Neumann sweeps' answer to b = 1, and K times it
     NdSystem &S = D.sys[0];
     DevBuf<double> w;
     rc = w.alloc(N) || S.kone.alloc(N) ? 100 : 0;
     if (!rc) {
-      k_nd_probe<<<nblk(N, 256), 256, 0, st>>>(N, pb, 0);
+      probe(kProbeOne);
       rc = nd_solve(h, 0, 1, pb, px, 1e-9, 1e-50, false);
     }
     if (!rc) {
@@ -1212,21 +1275,26 @@ static int nd_setup(nmg_handle *h, std::string &err) {
       S.one.swap(w);
     }
   }
-  // a system whose factor does not solve a probe to 1e-9 stays with the CG
-  k_nd_probe<<<nblk(N, 256), 256, 0, st>>>(N, pb, 1);
-  for (int mode = 0; mode < 2 && !rc; ++mode)
-    for (int f32 = 0; f32 < (h->mixed_cg() ? 2 : 1) && D.sys[mode].ready; ++f32) {
-      int flag = 0;
-      rc = nd_solve(h, mode, 1, pb, px, 1e-9, 1e-50, f32 == 1);
-      if (!rc && (cudaMemcpyAsync(&flag, W.err.p, sizeof(int), cudaMemcpyDeviceToHost, st) ||
-                  cudaStreamSynchronize(st)))
-        rc = 100;
-      if (rc || flag) {
-        D.sys[mode].ready = false;
-        cudaMemsetAsync(W.err.p, 0, sizeof(int), st);
-        nd_reset_barrier(h);
+  // a system whose factor does not solve the probes to the handle's tolerance,
+  // in fewer passes than a solve may take, stays with the CG
+  for (int kind = kProbeHash; kind < kProbes && !rc; ++kind) {
+    probe(kind);
+    for (int mode = 0; mode < 2 && !rc; ++mode)
+      for (int f32 = 0; f32 < (h->mixed_cg() ? 2 : 1) && D.sys[mode].ready; ++f32) {
+        int flag = 0, passes[2] = {0, 0};
+        rc = nd_solve(h, mode, 1, pb, px, std::min(1e-9, mode ? h->opt.dbc_rtol : h->opt.nbc_rtol), 1e-50, f32 == 1,
+                      NdOut(), true);
+        if (!rc && (cudaMemcpyAsync(&flag, W.err.p, sizeof(int), cudaMemcpyDeviceToHost, st) ||
+                    cudaMemcpyAsync(passes, W.iters.p, sizeof(passes), cudaMemcpyDeviceToHost, st) ||
+                    cudaStreamSynchronize(st)))
+          rc = 100;
+        if (rc || flag || passes[mode] > kNdProbePass) {
+          D.sys[mode].ready = false;
+          cudaMemsetAsync(W.err.p, 0, sizeof(int), st);
+          nd_reset_barrier(h);
+        }
       }
-    }
+  }
   W.iters.swap(iters);
   W.err.swap(errw);
   if (rc || cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
@@ -1258,7 +1326,7 @@ void nd_reset_barrier(nmg_handle *h) {
 }
 
 int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32,
-             const NdOut &out) {
+             const NdOut &out, bool probe) {
   NdSolver &D = h->nd;
   NdSystem &S = D.sys[mode];
   Workspace &W = h->ws;
@@ -1273,7 +1341,7 @@ int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double
   a.bar = D.bar; a.err = W.err; a.iters = W.iters;
   a.one = mode == 0 ? S.one.p : nullptr;
   a.kone = S.kone;
-  a.rtol = rtol; a.atol = atol;
+  a.rtol = rtol; a.atol = atol; a.probe = probe;
   void *args[] = {&a};
   const int mb = nd_members(nm);
   const void *fn = fp32 ? nd_kernel<float>(nm) : nd_kernel<double>(nm);

@@ -455,7 +455,7 @@ int nd_prepare(nmg_handle *h);
 bool nd_available(const nmg_handle *h, int mode);
 int post_fields(nmg_handle *h, double *fields, double *scalars);
 int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32,
-             const NdOut &out = NdOut());
+             const NdOut &out = NdOut(), bool probe = false);
 void nd_reset_barrier(nmg_handle *h);   // after a launch whose barrier gave up
 // ---- bem_tc.cu ----
 int bem_tc_setup(nmg_handle *h, std::string &err);
