@@ -13,7 +13,7 @@
 // swizzle).  The K dimension (the boundary nodes the matrix sums over) is
 // split over CTAs, each accumulating at most kKbPerSplit x 64 terms of every
 // sum in FP32 (the hi.hi term and the five smaller terms in two separate TMEM
-// accumulators); the per-split partial sums are added in FP32 pairs, in split
+// accumulators); the per-split partial sums are added to FP64's precision, in split
 // order, by a second kernel.  So the FP32 accumulation error stays at the
 // level of a thousand terms, not of nb.
 //
@@ -270,26 +270,34 @@ __global__ void __launch_bounds__(192, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
+// a + b rounded to FP32, and the rounding error (exact).
+__device__ __forceinline__ float two_sum(float a, float b, float &err) {
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+  return s;
+}
+
 // y[n * nb + row] = sum over the splits, in split order, of the FP32 partials.
-// The sum is kept as an FP32 pair (TwoSum, the rounding errors in the second
-// part: ~2^-47 of the terms, whose own error is 2^-24) and leaves as FP64: 21
-// conversions and FP64 adds per value made this FP64-pipe-bound (212 us for the
-// film's 128 vectors, 67 now; its 240 MB take 36).
+// The sum is kept in three FP32 numbers (the rounding errors of the first in
+// the second, those of the second in the third: ~2^-70 of the terms) and rounded
+// to FP64 once, so it is no further from the partials' sum than FP64 adds would
+// leave it: 21 conversions and FP64 adds per value made this FP64-pipe-bound (212
+// us for the film's 128 vectors, 67 now; its 240 MB take 36).
 __global__ void __launch_bounds__(256) k_tc_reduce(int nb, int Rpad, int Mpad, int splits,
                                                    const float *__restrict__ part, double *__restrict__ y) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x, n = blockIdx.y;
   if (row >= nb) return;
   const float *p = part + (size_t)n * Mpad + row;
   const size_t stride = (size_t)Rpad * Mpad;
-  float S = 0.f, C = 0.f;
+  float S = 0.f, C = 0.f, D = 0.f;
 #pragma unroll 8
   for (int k = 0; k < splits; ++k) {
-    const float v = __ldcs(p + k * stride);
-    const float s = __fadd_rn(S, v), b = __fsub_rn(s, S);
-    C = __fadd_rn(C, __fadd_rn(__fsub_rn(S, __fsub_rn(s, b)), __fsub_rn(v, b)));
-    S = s;
+    float e, f;
+    S = two_sum(S, __ldcs(p + k * stride), e);
+    C = two_sum(C, e, f);
+    D = __fadd_rn(D, f);
   }
-  double sum = (double)S + (double)C;
+  double sum = (double)S + ((double)C + (double)D);
   if (!isfinite(sum)) {   // beyond FP32's range, or not finite to begin with
     sum = 0.0;
     for (int k = 0; k < splits; ++k) sum += (double)p[k * stride];
