@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(256) k_fill_columns(FillArgs a) {
     const double gl = fma(g.gb, lm, fma(g.ga, ln, lv));
     // eta . (p_(v+1) - o), from differences of coordinates alone: with eta . p - eta . o
     // entries of an 18-unit box were off by 9e-14 of the largest at 1e4 from the origin, by 2e-12 at 4e5 (1e-15 so)
-    const double en = fma(g.eta[2], c2, fma(g.eta[1], c1, fma(g.eta[0], c0, g.height)));
+    const double en = fma(g.eta[0], c0, fma(g.eta[1], c1, fma(g.eta[2], c2, g.height)));
     acc = fma(g.fs, fma(angle, en, -(zeta * gl)), acc);
   }
   if (c == a.k0 + k) acc += a.solid_angle[c] / (4.0 * kPi) - 1.0;
