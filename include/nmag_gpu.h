@@ -195,7 +195,12 @@ int nmg_set_pinning(nmg_handle *h, const double *pin);
 
 /* Evaluate the RHS at the current m (program update_dmdt, nmag_lam.py:784-
  * 795) and copy fields out: fields = [H_exch | H_demag | H_anis | H_total |
- * dmdt] (5 x 3N), scalars = [phi | rho] (2 x N).  Either may be NULL. */
+ * dmdt] (5 x 3N), scalars = [phi | rho] (2 x N).  Either may be NULL.
+ * The Poisson systems are solved by CG until the solves of a handle, or those
+ * that an integration or an RK4 run is certain to make, are worth the
+ * factorisation, and directly from then on: each to the tolerances of the
+ * options, so that two evaluations of one m on either side of that differ by
+ * up to these (a direct answer is usually far closer). */
 int nmg_eval_fields(nmg_handle *h, double *fields, double *scalars);
 
 /* Energy densities [E_exch | E_demag | E_ext | E_anis | E_total] (5 x N) at

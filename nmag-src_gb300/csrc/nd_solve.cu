@@ -1304,21 +1304,67 @@ static int nd_setup(nmg_handle *h, std::string &err) {
   return 0;
 }
 
+// Iteration caps are the CG's: a caller that sets a small one, or chooses a
+// form of the CG's preconditioner, gets the CG.
+static bool nd_applies(const nmg_handle *h) {
+  const nmg_options &o = h->opt;
+  return o.do_demag && h->mesh.nb > 0 && !o.cg_no_coarse && o.cg_local_sweeps <= 1 && o.nbc_maxits >= kNdMinMaxits &&
+         o.dbc_maxits >= kNdMinMaxits;
+}
+
 int nd_prepare(nmg_handle *h) {
   if (h->pot) return nd_prepare(h->pot);   // several materials: the potential mesh's solves
   NdSolver &D = h->nd;
   if (D.tried) return 0;
   D.tried = true;
-  // Iteration caps are the CG's: a caller that sets a small one, or chooses a
-  // form of the CG's preconditioner, gets the CG.
-  const nmg_options &o = h->opt;
-  if (!o.do_demag || h->mesh.nb == 0 || o.cg_no_coarse || o.cg_local_sweeps > 1 || o.nbc_maxits < kNdMinMaxits ||
-      o.dbc_maxits < kNdMinMaxits)
-    return 0;
+  if (!nd_applies(h)) return 0;
   std::string err;
   const int rc = nd_setup(h, err);
   if (rc) h->last_error = err;
   return rc;
+}
+
+// Seconds of an iteration of the CG: grid barriers, which take longer with more
+// blocks, and a little for the nodes.  A fit (us measured, formula): 60 nodes 8.0
+// (8.2), 1,331 8.6 (8.9), slab of 11,163 10.9 (10.7), film of 30,753 12.7 (12.6),
+// cubes of 17,576 9.7 (11.4), 68,921 12.8 (14.8) and 132,651 19.4 (17.5).
+static double nd_iteration(const nmg_handle *h) { return 8e-6 + 2.6e-8 * std::sqrt((double)h->mesh.N); }
+
+// Seconds of nd_prepare, a fit to measured ones (ms, this formula in brackets):
+// 60 nodes 0.7 (1.2), 343 2.4 (2.1), 1,331 5.9 (5.9), slab of 11,163 14.5 (13.8),
+// box of 11,193 23 (23), film of 30,753 24 (29), cubes of 17,576 39 (36), 68,921
+// 158 (161) and 132,651 427 (382).  Thin meshes have small separators.
+static double nd_cost(const nmg_handle *h) {
+  const double N = h->mesh.N, in = N - h->mesh.nb;
+  return 1e-3 + 2.5e-6 * std::min(N, 2000.0) + 2e-6 * (N - 0.95 * h->mesh.nb) + 1e-11 * in * in;
+}
+
+int nd_note(nmg_handle *h) {
+  NdSolver &D = h->nd;
+  if (++D.evals < kNdEvals || D.tried) return 0;
+  if (!nd_applies(h)) return nd_prepare(h);
+  int total[2] = {0, 0};
+  if (cudaMemcpyAsync(total, h->ws.iters.p + 2, sizeof(total), cudaMemcpyDeviceToHost, h->stream) ||
+      cudaStreamSynchronize(h->stream)) {
+    h->last_error = "direct Poisson solver: reading the iteration counts failed";
+    return 100;
+  }
+  const double spent = ((double)total[0] + total[1]) * nd_iteration(h);
+  return spent + D.responses + D.certain >= kNdShare * nd_cost(h) ? nd_prepare(h) : 0;
+}
+
+int nd_response(nmg_handle *h) {
+  if (h->pot) return nd_response(h->pot);
+  NdSolver &D = h->nd;
+  D.responses += 2 * kNdResponseIters * nd_iteration(h);
+  return nd_note(h);
+}
+
+int nd_expect(nmg_handle *h, long long evals) {
+  if (h->pot) return nd_expect(h->pot, evals);
+  NdSolver &D = h->nd;
+  D.certain = std::max(D.certain, (double)evals * kNdIters * nd_iteration(h));
+  return !D.tried && nd_applies(h) && D.certain >= kNdShare * nd_cost(h) ? nd_prepare(h) : 0;
 }
 
 void nd_reset_barrier(nmg_handle *h) {

@@ -6,12 +6,18 @@ namespace nmg {
 
 // CG iteration caps below this keep the CG, whose cap they are.
 constexpr int kNdMinMaxits = 1000;
-// Demag evaluations after which a handle that has only evaluated fields gets
-// its factors: they cost as much as 6 to 15 evaluations save (film: 24 ms
-// against 3.2 ms each at 1e-12; cube: 6.5 ms against 1.1), so a program that
-// looks at one field does not pay for them.  Integrations, whose many
-// evaluations are certain, factor at their start.
+// A handle gets its factors once the CG's solves, those it has done and those
+// that are certain to come, are worth 3/4 of what the factors cost, so that a
+// program pays at most about twice what the better of the two would have taken,
+// whenever it stops.  Both are estimates, the same in every run: from the CG's
+// iteration counts, and from the mesh (nd_cost).  No handle is looked at before
+// its fourth demag evaluation.
 constexpr int kNdEvals = 4;
+constexpr double kNdShare = 0.75;
+// What is certain: an integration's first steps (64 evaluations; 100
+// iterations of the CG each, it takes 23 to 650), RK4's four evaluations a step.
+constexpr int kNdIntegration = 64, kNdIters = 100;
+constexpr int kNdResponseIters = 40;   // a Jacobian's demag response, solved to 1e-3
 
 struct NdFront {    // a part of the separator tree eliminated together
   int pos, k, nb, s;      // pivots [pos, pos + k) of the elimination order, boundary size, k + nb

@@ -210,6 +210,7 @@ struct NdSolver {
   NdSystem sys[2];                // 0: Neumann, 1: Dirichlet
   bool tried = false;             // nd_prepare has run
   int evals = 0;                  // demag evaluations so far
+  double certain = 0.0, responses = 0.0;   // seconds of CG to come, and spent on Jacobians' responses
   DevBuf<double> u, d, xw, r, part;   // member-minor work vectors, reduction partials
   DevBuf<unsigned> bar;           // barrier counter, blocks that left (both zero between launches)
 };
@@ -449,9 +450,14 @@ int jac_prepare(nmg_handle *P, JacDemag &J);
 int jac_demag_solve(nmg_handle *P, JacDemag &J, double rtol);
 // ---- nd_solve.cu (direct Poisson solves) ----
 // nd_prepare factors, once per handle, the systems the solver applies to
-// (nd_available); nd_solve: nm <= kChunk right-hand sides (member m at b + m * N)
+// (nd_available); nd_note, before each demag evaluation, nd_response, before a
+// Jacobian's, and nd_expect, where `evals` of them are certain, do so once it
+// is worth it; nd_solve: nm <= kChunk right-hand sides (member m at b + m * N)
 // to max(rtol |b|, atol).
 int nd_prepare(nmg_handle *h);
+int nd_note(nmg_handle *h);
+int nd_response(nmg_handle *h);
+int nd_expect(nmg_handle *h, long long evals);
 bool nd_available(const nmg_handle *h, int mode);
 int post_fields(nmg_handle *h, double *fields, double *scalars);
 int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32,

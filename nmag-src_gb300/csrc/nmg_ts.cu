@@ -1339,7 +1339,7 @@ void ts_destroy(Integrator *I) {
 
 int ts_init(nmg_handle *h, double t0) {
   Integrator &I = *h->ts;
-  if (int rc = nd_prepare(h)) return rc;
+  if (int rc = nd_expect(h, kNdIntegration)) return rc;
   I.tn = t0; I.q = 1; I.L = 2; I.qwait = I.L; I.qprime = 1;
   I.nst = I.nfe = I.nni = I.nli = I.ncfn = I.netf = I.nsetups = I.npe = I.nps = I.njv = 0;
   I.nstlp = I.nstlpre = 0;
@@ -1408,8 +1408,7 @@ int ts_advance(nmg_handle *h, double tout, int exact_tstop, int64_t max_steps, d
 // Classical RK4 with fixed dt on device vectors (differentiation form forward).
 int rk4_device(nmg_handle *h, double *d_m, double dt, int nsteps) {
   const int n = 3 * h->mesh.N * h->nrep;
-  if (nsteps > 0)
-    if (int rc = nd_prepare(h)) return rc;
+  if (int rc = nd_expect(h, 4LL * nsteps)) return rc;
   DevBuf<double> buf;
   if (buf.alloc(5 * (size_t)n)) return 100;
   double *k1 = buf.p, *k2 = k1 + n, *k3 = k2 + n, *k4 = k3 + n, *y = k4 + n;
@@ -1452,6 +1451,7 @@ int jacobian_apply(nmg_handle *h, const double *d_m, const double *d_v, double *
   JvArgs a = jv_base(h);
   a.mJ = d_m; a.HJ = h->ws.h_total; a.t = d_v; a.raw = 1; a.out = d_out;
   if (demag_in_jacobian(h)) {
+    if (int rc = nd_response(h)) return rc;
     if (demag_response(h, d_v)) return 100;
     a.hdv = h->jd.hdv;
   }

@@ -3180,8 +3180,10 @@ int check_device_error(nmg_handle *h, const char *where) {
 // potential W.phi: Neumann solve, boundary gather, BEM product, Dirichlet
 // load and solve, phi = phi1 + phi2 (nmag_lam.py:740-760).
 int demag_from_rho(nmg_handle *h) {
-  if (++h->nd.evals >= kNdEvals)
-    if (int rc = nd_prepare(h)) return rc;
+  // (not while a gradient's recomputation has to repeat its forward pass, nor
+  // within a Jacobian's response, whose tolerance is not the handle's)
+  if (!h->anchor_hold)
+    if (int rc = nd_note(h)) return rc;
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   cudaStream_t s = h->stream;

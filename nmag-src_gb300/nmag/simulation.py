@@ -139,6 +139,10 @@ class Simulation(object):
         self._do_demag = bool(do_demag)
         self.max_order = int(timestepper_max_order)
         self.krylov_max = int(timestepper_krylov_max)
+        # Poisson solves are iterative at first and direct once a simulation has
+        # made (or is certain to make) enough of them to pay for the
+        # factorisation, both to these tolerances (1e-5 by default): two
+        # evaluations of one m on either side of that differ by up to them
         self.ksp_tolerances = dict(ksp_tolerances or {})
         self.quirks = quirks
         self.bem_precision = bem_precision
