@@ -703,7 +703,7 @@ int rk4_forward(nmg_handle *h, const double *d_m0, double dt, int nsteps, int ck
     h->last_error = "the RK4 adjoint does not take a pinning field";
     return -2;
   }
-  if (int rc = nd_prepare(h)) return rc;   // now: the adjoint recomputes this pass with the same solver
+  if (int rc = nd_prepare(h, true)) return rc;   // now: the adjoint recomputes this pass with the same solver
   if (!h->tape) h->tape = new Tape();
   Tape &T = *h->tape;
   const bool same = T.n3 == n3 && T.ckpt == ckpt && T.nsteps == nsteps && T.npulses == npulses;

@@ -1169,8 +1169,7 @@ static int nd_build(nmg_handle *h, int mode, const std::vector<int32_t> &rp, con
       Dn.alloc((size_t)nfmax * kNdPanel * kNdPanel)) {
     cudaGetLastError();
     cudaStreamSynchronize(st);
-    S.f64.release();
-    S.f32.release();
+    S.release();
     return 0;   // no room: the CG needs less
   }
   if (n > 0)
@@ -1207,9 +1206,13 @@ static int nd_build(nmg_handle *h, int mode, const std::vector<int32_t> &rp, con
   return 0;
 }
 
-bool nd_available(const nmg_handle *h, int mode) { return h->nd.sys[mode].ready; }
+bool nd_available(const nmg_handle *h, int mode, bool fp32) {
+  const NdSystem &S = h->nd.sys[mode];
+  return S.ready && (S.n == 0 || (fp32 ? S.f32.p != nullptr : S.f64.p != nullptr));   // (n = 0: nothing but the boundary)
+}
 
-static int nd_setup(nmg_handle *h, std::string &err) {
+// with64: FP64 factors stay beside (or in place of) the FP32 ones.
+static int nd_setup(nmg_handle *h, bool with64, std::string &err) {
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   NdSolver &D = h->nd;
@@ -1233,7 +1236,7 @@ static int nd_setup(nmg_handle *h, std::string &err) {
       D.r.alloc((size_t)N * MB) || D.part.alloc(2 * 2 * (size_t)kChunk * h->sm_count) || D.bar.alloc(2) ||
       pb.alloc(N) || px.alloc(N) || iters.alloc(4) || errw.alloc(1)) {
     cudaGetLastError();   // no room: the CG needs less
-    D.sys[0].ready = D.sys[1].ready = false;
+    D.release();
     return 0;
   }
   NMG_CUDA_TRY(cudaMemsetAsync(D.bar.p, 0, 2 * sizeof(unsigned), st), "memset");
@@ -1289,7 +1292,7 @@ static int nd_setup(nmg_handle *h, std::string &err) {
                     cudaStreamSynchronize(st)))
           rc = 100;
         if (rc || flag || passes[mode] > kNdProbePass) {
-          D.sys[mode].ready = false;
+          D.sys[mode].release();
           cudaMemsetAsync(W.err.p, 0, sizeof(int), st);
           nd_reset_barrier(h);
         }
@@ -1301,6 +1304,9 @@ static int nd_setup(nmg_handle *h, std::string &err) {
     err = "direct Poisson solver: setup failed";
     return 100;
   }
+  if (!with64)
+    for (NdSystem &s : D.sys) s.f64.release();
+  if (!D.sys[0].ready && !D.sys[1].ready) D.release();
   return 0;
 }
 
@@ -1312,16 +1318,33 @@ static bool nd_applies(const nmg_handle *h) {
          o.dbc_maxits >= kNdMinMaxits;
 }
 
-int nd_prepare(nmg_handle *h) {
-  if (h->pot) return nd_prepare(h->pot);   // several materials: the potential mesh's solves
+int nd_prepare(nmg_handle *h, bool adjoint) {
+  if (h->pot) return nd_prepare(h->pot, adjoint);   // several materials: the potential mesh's solves
   NdSolver &D = h->nd;
-  if (D.tried) return 0;
+  const nmg_options &o = h->opt;
+  // who solves in FP64; the other handles keep the FP32 factors alone
+  const bool with64 = D.with64 || o.cg_precision != 1 || (adjoint && o.adjoint_cg_precision != 1);
+  if (D.tried && with64 == D.with64) return 0;
+  const bool again = D.tried && (D.sys[0].ready || D.sys[1].ready);
+  if (!nd_applies(h) || (D.tried && !again)) {
+    D.tried = true;
+    D.with64 = with64;
+    return 0;
+  }
+  D.release();
   D.tried = true;
-  if (!nd_applies(h)) return 0;
+  D.with64 = with64;
   std::string err;
-  const int rc = nd_setup(h, err);
-  if (rc) h->last_error = err;
-  return rc;
+  if (nd_setup(h, with64, err)) {
+    // refused by the device: nothing is kept, and the CG answers, if the device still does
+    D.release();
+    cudaGetLastError();
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
+      h->last_error = err;
+      return 100;
+    }
+  }
+  return 0;
 }
 
 // Seconds of an iteration of the CG: grid barriers, which take longer with more

@@ -205,14 +205,27 @@ struct NdSystem {
   DevBuf<int32_t> bnd, map, perm, prow, pcol;   // perm: position of each node (-1: fixed), then node of each position
   DevBuf<double> pK, f64, one, kone;   // one, kone: the Neumann sweeps' answer to b = 1 and K times it
   DevBuf<float> f32;
+  void release() {
+    ready = false;
+    front.release(); phase.release(); task.release();
+    for (DevBuf<int32_t> *b : {&bnd, &map, &perm, &prow, &pcol}) b->release();
+    for (DevBuf<double> *b : {&pK, &f64, &one, &kone}) b->release();
+    f32.release();
+  }
 };
 struct NdSolver {
   NdSystem sys[2];                // 0: Neumann, 1: Dirichlet
   bool tried = false;             // nd_prepare has run
+  bool with64 = false;            // and kept FP64 factors
   int evals = 0;                  // demag evaluations so far
   double certain = 0.0, responses = 0.0;   // seconds of CG to come, and spent on Jacobians' responses
   DevBuf<double> u, d, xw, r, part;   // member-minor work vectors, reduction partials
   DevBuf<unsigned> bar;           // barrier counter, blocks that left (both zero between launches)
+  void release() {
+    for (NdSystem &s : sys) s.release();
+    for (DevBuf<double> *b : {&u, &d, &xw, &r, &part}) b->release();
+    bar.release();
+  }
 };
 
 // Several magnetic materials (nmag_lam.py:183-330): every material X has its
@@ -454,11 +467,11 @@ int jac_demag_solve(nmg_handle *P, JacDemag &J, double rtol);
 // Jacobian's, and nd_expect, where `evals` of them are certain, do so once it
 // is worth it; nd_solve: nm <= kChunk right-hand sides (member m at b + m * N)
 // to max(rtol |b|, atol).
-int nd_prepare(nmg_handle *h);
+int nd_prepare(nmg_handle *h, bool adjoint = false);   // adjoint: also what its solves need
 int nd_note(nmg_handle *h);
 int nd_response(nmg_handle *h);
 int nd_expect(nmg_handle *h, long long evals);
-bool nd_available(const nmg_handle *h, int mode);
+bool nd_available(const nmg_handle *h, int mode, bool fp32);
 int post_fields(nmg_handle *h, double *fields, double *scalars);
 int nd_solve(nmg_handle *h, int mode, int nm, const double *b, double *x, double rtol, double atol, bool fp32,
              const NdOut &out = NdOut(), bool probe = false);

@@ -2583,7 +2583,7 @@ void wait_basis_factor(nmg_handle *h, int ev_slot) {
 // `out` (the direct solves alone): what else is written with the answer.
 int run_cg(nmg_handle *h, int mode, const double *b, double *x, double rtol, double atol, int maxits,
            const NdOut &out = NdOut()) {
-  if (nd_available(h, mode & 1)) return nd_solve(h, mode & 1, 1, b, x, rtol, atol, false, out);
+  if (nd_available(h, mode & 1, false)) return nd_solve(h, mode & 1, 1, b, x, rtol, atol, false, out);
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   CGArgs a;
@@ -2627,8 +2627,8 @@ int run_cg(nmg_handle *h, int mode, const double *b, double *x, double rtol, dou
 // mixed precision, 0 FP64, -1 the handle's forward choice.
 int run_cgm(nmg_handle *h, int mode, int c0, const double *b, double *x, int nm, double rtol, double atol,
             int maxits, int bslot = -1, int mp_sel = -1, const NdOut &out = NdOut()) {
-  if (nd_available(h, mode))
-    return nd_solve(h, mode, nm, b, x, rtol, atol, mp_sel >= 0 ? mp_sel == 1 : h->opt.cg_precision == 1, out);
+  const bool fp32 = mp_sel >= 0 ? mp_sel == 1 : h->opt.cg_precision == 1;
+  if (nd_available(h, mode, fp32)) return nd_solve(h, mode, nm, b, x, rtol, atol, fp32, out);
   Mesh &M = h->mesh;
   Workspace &W = h->ws;
   CGArgs a;
@@ -3190,7 +3190,7 @@ int demag_from_rho(nmg_handle *h) {
   const int N = M.N;
   const int B = h->nrep;
   // the direct solves write the boundary values and phi1 + phi2 themselves
-  const bool nd0 = nd_available(h, 0), nd1 = nd_available(h, 1);
+  const bool fp32 = h->opt.cg_precision == 1, nd0 = nd_available(h, 0, fp32), nd1 = nd_available(h, 1, fp32);
   auto out = [&](int mode, int c0) {
     NdOut o;
     if (mode == 0) o.bnd = W.b1.p + (size_t)c0 * M.nb;
