@@ -35,9 +35,11 @@ struct DevBuf {
   DevBuf &operator=(const DevBuf &) = delete;
   cudaError_t alloc(size_t count) {
     release();
-    n = count;
     if (!count) return cudaSuccess;
-    return cudaMalloc(&p, sizeof(T) * count);
+    const cudaError_t e = cudaMalloc(&p, sizeof(T) * count);
+    if (e == cudaSuccess) n = count;
+    else p = nullptr;
+    return e;   // refused: an empty buffer, of size 0
   }
   void release() {
     if (p) cudaFree(p);
