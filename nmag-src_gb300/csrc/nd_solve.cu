@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(kNdThreads, 1) k_nd_solve(NdArgs a) {
   if (a.nlev == 0) nd_arrive(a);
 
   int pass = 0;
-  bool failed = false;
+  int failed = 0;
   // the vector entry a task's row products need at local index c of front f:
   // right-hand side plus the children's u (c < k), the solution's negative
   // (downwards, c >= k)
@@ -824,7 +824,7 @@ __global__ void __launch_bounds__(kNdThreads, 1) k_nd_solve(NdArgs a) {
     if (!nd_wait(a, epoch)) return;
     nd_total<MB>(slot1, s_res);
     if (tid == 0) {
-      int st = 1;   // 1 done, 0 another pass, 2 failed, 3 done if what is left is rounding
+      int st = 1;   // 1 done, 0 another pass, 2 not finite, 3 done if what is left is rounding
       for (int m = 0; m < a.nm; ++m) {
         const double rn = sqrt(s_res[m]);
         if (!(rn == rn) || isinf(rn)) st = 2;
@@ -869,9 +869,9 @@ __global__ void __launch_bounds__(kNdThreads, 1) k_nd_solve(NdArgs a) {
       __syncthreads();
       st = s_state;
     }
-    if (st == 0 && pass + 1 >= kNdMaxPass) st = 2;
-    failed = st == 2;
-    if (st != 0) break;
+    if (st == 2) failed = ERR_NONFINITE;
+    else if (st == 0 && pass + 1 >= kNdMaxPass) failed = ERR_CG_MAXITS;
+    if (st != 0 || failed) break;
     nd_arrive(a);   // slot1 is free, r is complete
   }
   {
@@ -898,7 +898,7 @@ __global__ void __launch_bounds__(kNdThreads, 1) k_nd_solve(NdArgs a) {
   if (gt == 0) {
     a.iters[a.mode] = pass + 1;
     a.iters[2 + a.mode] += pass + 1;
-    if (failed) atomicOr(a.err, ERR_CG_MAXITS);
+    if (failed) atomicOr(a.err, failed);
   }
   nd_leave(a);
 }

@@ -18,7 +18,7 @@ enum DeviceError : int {
   ERR_DEGREE = 1,       // a node belongs to more tets than the fixed-size row buffer allows
   ERR_BARRIER = 2,      // a grid barrier gave up waiting (bounded spin)
   ERR_NONFINITE = 4,    // a solver produced NaN/Inf
-  ERR_CG_MAXITS = 8,    // CG hit its iteration cap
+  ERR_CG_MAXITS = 8,    // a Poisson solve hit its cap (CG iterations, passes over the factors)
 };
 
 constexpr int kMaxRowLen = 64;     // max distinct neighbours (incl. self) per node

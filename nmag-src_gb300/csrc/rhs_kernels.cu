@@ -3169,7 +3169,7 @@ int check_device_error(nmg_handle *h, const char *where) {
     if (derr & ERR_BARRIER) nd_reset_barrier(h);
     if (derr & ERR_BARRIER) h->last_error = std::string(where) + ": grid barrier timed out";
     else if (derr & ERR_NONFINITE) h->last_error = std::string(where) + ": solver produced non-finite values";
-    else if (derr & ERR_CG_MAXITS) h->last_error = std::string(where) + ": CG reached its iteration limit";
+    else if (derr & ERR_CG_MAXITS) h->last_error = std::string(where) + ": a Poisson solve reached its iteration limit";
     else h->last_error = std::string(where) + ": device error flag " + std::to_string(derr);
     return (derr & ERR_BARRIER) ? 7 : ((derr & ERR_NONFINITE) ? 6 : 5);
   }
