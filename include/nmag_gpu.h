@@ -394,7 +394,8 @@ int nmg_batch_eval(nmg_batch *b, double *dmdt, double *h_total);
 int nmg_batch_run(nmg_batch *b, int launches);
 int nmg_batch_state(const nmg_batch *b, double *t, int32_t *stage, int64_t *steps, int64_t *rhs_evals,
                     int32_t *done, double *max_dmdt);
-/* CTA size and per-launch work budget; the autotuner times candidates on the
+/* CTA size (a multiple of 32; the kernel's registers allow up to 352) and
+ * per-launch work budget; a size that is refused changes nothing.  The autotuner times candidates on the
  * batch (state restored afterwards) and keeps the fastest. */
 int nmg_batch_set_schedule(nmg_batch *b, int threads, double budget);
 int nmg_batch_autotune(nmg_batch *b, int trial_launches, int *threads_out, double *budget_out);
