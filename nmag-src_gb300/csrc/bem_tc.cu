@@ -282,7 +282,8 @@ __device__ __forceinline__ float two_sum(float a, float b, float &err) {
 // the second, those of the second in the third: ~2^-70 of the terms) and rounded
 // to FP64 once, so it is no further from the partials' sum than FP64 adds would
 // leave it: 21 conversions and FP64 adds per value made this FP64-pipe-bound (212
-// us for the film's 128 vectors, 67 now; its 240 MB take 36).
+// us for the film's 128 vectors, 67 with two FP32 numbers, and the whole product
+// takes 592 us with either two or three; its 240 MB take 36).
 __global__ void __launch_bounds__(256) k_tc_reduce(int nb, int Rpad, int Mpad, int splits,
                                                    const float *__restrict__ part, double *__restrict__ y) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x, n = blockIdx.y;

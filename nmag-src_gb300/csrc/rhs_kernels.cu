@@ -2314,7 +2314,6 @@ __global__ void k_energy(int N, const double *__restrict__ m, const double *__re
   E[4 * (size_t)N + i] = ((dm + ex) + ez) + an;
 }
 
-// Block partial sums of V_i, V_i m_i (3) and V_i E_k,i (5): 9 columns.
 // The block that finishes last goes on to add the blocks' partials.
 __device__ __forceinline__ bool last_block(unsigned *count) {
   __shared__ bool last;
@@ -2329,6 +2328,8 @@ __device__ __forceinline__ bool last_block(unsigned *count) {
   return last;
 }
 constexpr int kAvgBlocks = 64;   // two partials a lane in the last block
+// Sums of V_i, V_i m_i (3) and V_i E_k,i (5): 9 columns of block partials, added
+// by the last block and posted to the host.
 __global__ void k_avg(int N, const double *__restrict__ m, const double *__restrict__ vol,
                       const double *__restrict__ E, double *part, size_t estride, unsigned *count, double *host,
                       unsigned long long *flag, unsigned long long seq) {
