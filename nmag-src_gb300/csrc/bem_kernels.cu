@@ -35,6 +35,7 @@
 #include <cmath>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "nmg_internal.h"
@@ -155,7 +156,11 @@ struct FillArgs {
   const TriGeo *geo;
   const VertexGeo *vgeo;
   double *dist, *lg, *ang, *zeta, *bem;
+  int *touch;   // set where an observer lies on an edge, or next to it
 };
+// The upper words of 28 and of infinity.  A logarithm of 28 or more: (a + b - s) / s
+// below 1.4e-12, infinite or not a number.
+constexpr unsigned k28 = 0x403c0000u, kInf = 0x7ff00000u;
 
 // Distance of every boundary node from every observer of the chunk.
 __global__ void __launch_bounds__(256) k_fill_dist(FillArgs a) {
@@ -178,7 +183,8 @@ template <bool kExact>
 __global__ void __launch_bounds__(256) k_fill_edges(FillArgs a) {
   const int k = blockIdx.x * 32 + (threadIdx.x & 31), e = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (k >= a.kc || e >= a.ne || a.k0 + k >= a.nb) return;
-  const double L = a.dist[(size_t)a.edge[2 * e] * a.kc + k] + a.dist[(size_t)a.edge[2 * e + 1] * a.kc + k];
+  const double da = a.dist[(size_t)a.edge[2 * e] * a.kc + k], db = a.dist[(size_t)a.edge[2 * e + 1] * a.kc + k];
+  const double L = da + db;
   const double s = a.edge_len[e];
   double v;
   if (!kExact && 8.0 * s <= L) {
@@ -189,6 +195,7 @@ __global__ void __launch_bounds__(256) k_fill_edges(FillArgs a) {
     v = 2.0 * fma(x * y, t, x);
   } else {
     v = log((L + s) / (L - s));
+    if ((unsigned)__double2hiint(v) >= k28 && da != 0.0 && db != 0.0) *a.touch = 1;   // (not an end of the edge)
   }
   a.lg[(size_t)e * a.kc + k] = v;
 }
@@ -197,8 +204,10 @@ __global__ void __launch_bounds__(256) k_fill_edges(FillArgs a) {
 // infinite: the triangle adds nothing (degenerate, the observer one of its
 // vertices or in its plane, bem3d_stubs.c:531-600).  In the plane the reference
 // adds 0 times the formula, which is not a number where the observer lies on an
-// edge (a node on another part's edge): such an entry stays NaN, to be noticed.
-template <bool kExact>
+// edge (a node on another part's edge): with kTouch such an entry stays NaN, to
+// be noticed.  (Looking for it in every triangle of an observer's plane took 1 to
+// 2 of the 57 ms of an 8,562-node handle; k_fill_edges tells which mesh needs it.)
+template <bool kExact, bool kTouch>
 __global__ void __launch_bounds__(256) k_fill_angles(FillArgs a) {
   const int k = blockIdx.x * 32 + (threadIdx.x & 31), t = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (k >= a.kc || t >= a.ntri || a.k0 + k >= a.nb) return;
@@ -216,18 +225,14 @@ __global__ void __launch_bounds__(256) k_fill_angles(FillArgs a) {
   const double zeta = g.zeta_v[0] * r[0][0] + g.zeta_v[1] * r[0][1] + g.zeta_v[2] * r[0][2];
   const double geo_eps = (g.maxgeo > omax ? g.maxgeo : omax) * 1e-13;
   const bool plane = fabs(zeta) < geo_eps;
-  // In the plane: on an edge or next to it (its logarithm 28 or more, (a + b - s) / s
-  // below 1.4e-12, infinite or not a number); the formula is finite elsewhere.  The
-  // upper words alone: FP64 comparisons here cost a handle of 8,562 nodes 2 of 57 ms.
-  auto edge = [&](unsigned least) {
+  auto edge = [&](unsigned least) {   // on an edge or next to it: elsewhere in the plane the formula is finite
     const int32_t *te = a.tri_edge + 3 * (size_t)t;
     bool any = false;
 #pragma unroll
     for (int v = 0; v < 3; ++v) any |= (unsigned)__double2hiint(a.lg[(size_t)te[v] * a.kc + k]) >= least;
     return any;
   };
-  constexpr unsigned k28 = 0x403c0000u, kInf = 0x7ff00000u;
-  if (g.ok && !(rl[0] <= 0.0 || rl[1] <= 0.0 || rl[2] <= 0.0) && (!plane || edge(k28))) {
+  if (g.ok && !(rl[0] <= 0.0 || rl[1] <= 0.0 || rl[2] <= 0.0) && (!plane || (kTouch && edge(k28)))) {
     const double sp01 = r[0][0] * r[1][0] + r[0][1] * r[1][1] + r[0][2] * r[1][2];
     const double sp12 = r[1][0] * r[2][0] + r[1][1] * r[2][1] + r[1][2] * r[2][2];
     const double sp20 = r[2][0] * r[0][0] + r[2][1] * r[0][1] + r[2][2] * r[0][2];
@@ -247,7 +252,7 @@ __global__ void __launch_bounds__(256) k_fill_angles(FillArgs a) {
         angle = 2.0 * acos(q);
       }
       if (zeta < 0.0) angle = -angle;
-      if (plane) angle = angle != angle || edge(kInf) ? nan("") : kNothing;
+      if (kTouch && plane) angle = angle != angle || edge(kInf) ? nan("") : kNothing;
     }
   }
   a.ang[(size_t)t * a.kc + k] = angle;
@@ -446,19 +451,29 @@ int fill_bem(nmg_handle *h, std::string &err, bool exact) {
       err = "BEM fill: surface too large (more than 524,280 nodes, edges or triangles)";
       return 3;
     }
-    for (a.k0 = 0; a.k0 < M.nb; a.k0 += kc) {
-      const unsigned gx = (unsigned)((std::min(kc, M.nb - a.k0) + 31) / 32);
-      k_fill_dist<<<dim3(gx, (M.nb + 7) / 8), 256, 0, s>>>(a);
-      const dim3 ge(gx, (ne + 7) / 8), gt(gx, (nt + 7) / 8), gc(gx, (M.nb + 7) / 8);
-      if (exact) {
-        if (ne > 0) k_fill_edges<true><<<ge, 256, 0, s>>>(a);
-        if (nt > 0) k_fill_angles<true><<<gt, 256, 0, s>>>(a);
-        k_fill_columns<true><<<gc, 256, 0, s>>>(a);
-      } else {
-        if (ne > 0) k_fill_edges<false><<<ge, 256, 0, s>>>(a);
-        if (nt > 0) k_fill_angles<false><<<gt, 256, 0, s>>>(a);
-        k_fill_columns<false><<<gc, 256, 0, s>>>(a);
+    DevBuf<int> touch;
+    NMG_CUDA_TRY(touch.alloc(1), "alloc");
+    NMG_CUDA_TRY(cudaMemsetAsync(touch.p, 0, sizeof(int), s), "memset");
+    a.touch = touch;
+    auto fill = [&](auto ex, auto touching) {
+      constexpr bool kExact = decltype(ex)::value, kTouch = decltype(touching)::value;
+      for (a.k0 = 0; a.k0 < M.nb; a.k0 += kc) {
+        const unsigned gx = (unsigned)((std::min(kc, M.nb - a.k0) + 31) / 32);
+        const dim3 ge(gx, (ne + 7) / 8), gt(gx, (nt + 7) / 8), gc(gx, (M.nb + 7) / 8);
+        k_fill_dist<<<gc, 256, 0, s>>>(a);
+        if (ne > 0) k_fill_edges<kExact><<<ge, 256, 0, s>>>(a);
+        if (nt > 0) k_fill_angles<kExact, kTouch><<<gt, 256, 0, s>>>(a);
+        k_fill_columns<kExact><<<gc, 256, 0, s>>>(a);
       }
+    };
+    if (exact) fill(std::true_type(), std::false_type());
+    else fill(std::false_type(), std::false_type());
+    int touching = 0;   // parts that touch with unlike cells, which is rare: once more, looking at edges
+    NMG_CUDA_TRY(cudaMemcpyAsync(&touching, touch.p, sizeof(int), cudaMemcpyDeviceToHost, s), "d2h");
+    NMG_CUDA_TRY(cudaStreamSynchronize(s), "bem fill");
+    if (touching) {
+      if (exact) fill(std::true_type(), std::true_type());
+      else fill(std::false_type(), std::true_type());
     }
     NMG_CUDA_TRY(cudaGetLastError(), "bem fill launch");
     NMG_CUDA_TRY(M.bem.alloc(nb * M.ld), "alloc BEM (nb x ld doubles)");
